@@ -265,6 +265,16 @@ typedef struct rt_launch_opts {
 rt_status rt_matmul_launch_ex(rt_plan *plan, const void *lhs, const void *rhs, const void *bias, void *out, void *stream,
                               const rt_launch_opts *opts);
 
+/* A number for the present values of the environment switches that change which kernel rt_matmul_plan picks: a caller
+ * that keeps plans beside its own node descriptions plans again when it changes. */
+uint64_t rt_routing_stamp(void);
+/* Tensor::resolve's dispatch loop (tensor.rs:738-787) in one call: n nodes in execution order, each with a new output buffer
+ * from the device's pool, launched on the device's stream.  Node i is five words at nodes[5 i]: the plan, the device
+ * pointers of lhs, rhs and bias (0: none), the launch flags; an odd pointer word 2 k + 1 is the output of node k < i.  For
+ * each node outs[3 i] gets the rt_buffer *, its device pointer and its size; *n_done is how many nodes were launched
+ * (fewer than n only with an error; the buffers of those are the caller's). */
+rt_status rt_graph_resolve(rt_device *dev, const uint64_t *nodes, int32_t n, uint64_t *outs, int32_t *n_done);
+
 /* One dispatch: the operands of one planned node. */
 typedef struct rt_dispatch {
     rt_plan *plan;

@@ -166,6 +166,8 @@ def load() -> ctypes.CDLL:
         "rt_plan_launches": (c_int32, [V]),
         "rt_matmul_launch": (c_int32, [V, V, V, V, V, V]),
         "rt_matmul_launch_ex": (c_int32, [V, V, V, V, V, V, POINTER(rt_launch_opts)]),
+        "rt_routing_stamp": (c_uint64, []),
+        "rt_graph_resolve": (c_int32, [V, POINTER(c_uint64), c_int32, POINTER(c_uint64), POINTER(c_int32)]),
         "rt_executable_create": (c_int32, [V, POINTER(rt_dispatch), c_int32, c_int32, POINTER(V)]),
         "rt_executable_create_planned": (c_int32, [V, POINTER(rt_dispatch), POINTER(rt_node_tensors), c_int32,
                                                    POINTER(c_uint64), c_int32, c_int32, POINTER(V)]),

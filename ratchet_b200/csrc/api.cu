@@ -48,6 +48,8 @@ struct rt_device {
     std::unordered_map<std::string, rt_plan *> plans;
     std::mutex kept_mu;
     std::unordered_map<const void *, int> kept_ptrs; // weight pointers some plan keeps a dequantised copy of
+    std::mutex stage_mu;
+    void *stage = nullptr; // page-locked, STAGE_BYTES: small results on their way to pageable memory
 };
 
 static inline uint64_t size_class(uint64_t n) {
@@ -118,6 +120,53 @@ struct rt_plan {
     }
 };
 
+// The kernel families that report a bounded wait which ran out (wait_error.cuh), and what the host says of it.
+struct WaitFamily {
+    cudaError_t (*bind)(int *word);
+    const char *what, *left;
+};
+static const WaitFamily WAIT_FAMILIES[] = {
+    {umma_bind_wait_error, "a tensor-core GEMM", "its output is incomplete"},
+    {umma_tf32_bind_wait_error, "an f32 tensor-core GEMM", "its output is incomplete"},
+    {gemv_umma_bind_wait_error, "a tensor-memory GEMV", "its output is incomplete"},
+    {gemv_chain_bind_wait_error, "a GEMV chain", "its outputs are incomplete"},
+    {gemv_q4k_bind_wait_error, "a Q4_K GEMV", "its output is incomplete"},
+    {gemv_q4k_umma_bind_wait_error, "a tensor-memory Q4_K GEMV", "its output is incomplete"},
+    {gemv_bind_wait_error, "a GEMV", "its output is incomplete"},
+};
+constexpr int N_WAIT_FAMILIES = (int)(sizeof(WAIT_FAMILIES) / sizeof(WAIT_FAMILIES[0]));
+constexpr int MAX_ORDINALS = 64;
+static std::mutex g_wait_words_mu;
+static int *g_wait_words[MAX_ORDINALS]; // one word per family, page-locked, for the life of the process
+
+static int *wait_words(int ordinal) { return ordinal >= 0 && ordinal < MAX_ORDINALS ? g_wait_words[ordinal] : nullptr; }
+
+// Once per ordinal (the current device), before any handle on it exists.
+static cudaError_t bind_wait_words(int ordinal) {
+    std::lock_guard<std::mutex> lk(g_wait_words_mu);
+    if (ordinal >= MAX_ORDINALS || g_wait_words[ordinal]) return cudaSuccess;
+    int *words = nullptr;
+    cudaError_t e = cudaHostAlloc((void **)&words, sizeof(int) * N_WAIT_FAMILIES, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    memset(words, 0, sizeof(int) * N_WAIT_FAMILIES);
+    for (int f = 0; f < N_WAIT_FAMILIES && e == cudaSuccess; f++) e = WAIT_FAMILIES[f].bind(words + f);
+    if (e == cudaSuccess) g_wait_words[ordinal] = words;
+    return e; // (on failure the words stay allocated: some family may already hold theirs)
+}
+
+// The environment switches that change which kernel a plan takes.
+static const char *const ROUTING_SWITCHES[] = {"RT_FORCE_KERNEL", "RT_GEMV_UMMA", "RT_Q4K_UMMA", "RT_GEMM_PAIR", "RT_GEMM_PAIR_MIN",
+                                               "RT_TF32_BN", "RT_TF32_PRESPLIT", "RT_Q4K_WALK_FROM", "RT_KEEP_WEIGHTS"};
+static std::string routing_switches() {
+    std::string k;
+    for (const char *name : ROUTING_SWITCHES) {
+        const char *v = getenv(name);
+        k += '|';
+        if (v) k += v;
+    }
+    return k;
+}
+
 // Everything of a node description that routing looks at, field by field (the struct has padding bytes), plus the
 // debugging switches that change routing.
 static std::string plan_key(const rt_matmul_desc &d) {
@@ -131,11 +180,7 @@ static std::string plan_key(const rt_matmul_desc &d) {
     put_shape(d.lhs_shape); put_shape(d.rhs_shape);
     if (d.has_bias) put_shape(d.bias_shape);
     put(d.has_bias != 0); put(d.trans_lhs != 0); put(d.trans_rhs != 0); put(d.trans_out != 0); put(d.epilogue);
-    for (const char *name : {"RT_FORCE_KERNEL", "RT_GEMV_UMMA", "RT_Q4K_UMMA", "RT_GEMM_PAIR", "RT_GEMM_PAIR_MIN", "RT_TF32_BN", "RT_TF32_PRESPLIT", "RT_Q4K_WALK_FROM", "RT_KEEP_WEIGHTS"}) {
-        const char *v = getenv(name);
-        k += '|';
-        if (v) k += v;
-    }
+    k += routing_switches();
     return k;
 }
 
@@ -341,6 +386,7 @@ rt_status rt_device_create(int32_t ordinal, rt_device **dev) {
         return fail(RT_ERR_UNSUPPORTED, std::string("device ") + prop.name + " is sm_" + std::to_string(prop.major) +
                                             std::to_string(prop.minor) + "; the kernels are built for sm_100a only");
     CUDA_TRY(cudaSetDevice(ordinal));
+    CUDA_TRY(bind_wait_words(ordinal));
     rt_device *d = new (std::nothrow) rt_device();
     if (!d) return fail(RT_ERR_NOMEM, "out of host memory");
     d->ordinal = ordinal;
@@ -365,6 +411,7 @@ rt_status rt_device_destroy(rt_device *dev) {
     dev->plans.clear();
     for (auto &kv : dev->pool)
         for (void *p : kv.second) cudaFree(p);
+    if (dev->stage) cudaFreeHost(dev->stage);
     if (dev->stream) cudaStreamDestroy(dev->stream);
     delete dev;
     return RT_OK;
@@ -374,27 +421,13 @@ rt_status rt_device_sync(rt_device *dev) {
     if (!dev) return fail(RT_ERR_ARG, "rt_device_sync: null device");
     CUDA_TRY(cudaSetDevice(dev->ordinal));
     CUDA_TRY(cudaStreamSynchronize(dev->stream));
-    int site = 0;
-    CUDA_TRY(umma_take_error(&site, dev->stream));
-    if (site != 0)
-        return fail(RT_ERR_CUDA, "a tensor-core GEMM gave up a bounded wait (site " + std::to_string(site) +
-                                     "): its output is incomplete");
-    CUDA_TRY(umma_tf32_take_error(&site, dev->stream));
-    if (site != 0)
-        return fail(RT_ERR_CUDA, "an f32 tensor-core GEMM gave up a bounded wait (site " + std::to_string(site) + "): its output is incomplete");
-    CUDA_TRY(gemv_umma_take_error(&site, dev->stream));
-    if (site != 0)
-        return fail(RT_ERR_CUDA, "a tensor-memory GEMV gave up a bounded wait (site " + std::to_string(site) + "): its output is incomplete");
-    CUDA_TRY(gemv_chain_take_error(&site, dev->stream));
-    if (site != 0)
-        return fail(RT_ERR_CUDA, "a GEMV chain gave up a bounded wait (site " + std::to_string(site) + "): its outputs are incomplete");
-    CUDA_TRY(gemv_q4k_take_error(&site, dev->stream));
-    if (site != 0) return fail(RT_ERR_CUDA, "a Q4_K GEMV gave up waiting for its weight copies: its output is incomplete");
-    CUDA_TRY(gemv_q4k_umma_take_error(&site, dev->stream));
-    if (site != 0)
-        return fail(RT_ERR_CUDA, "a tensor-memory Q4_K GEMV gave up a bounded wait (site " + std::to_string(site) + "): its output is incomplete");
-    CUDA_TRY(gemv_take_error(&site, dev->stream));
-    if (site != 0) return fail(RT_ERR_CUDA, "a GEMV gave up waiting for its weight copies: its output is incomplete");
+    volatile int *const words = wait_words(dev->ordinal);
+    for (int f = 0; words && f < N_WAIT_FAMILIES; f++) {
+        const int site = words[f];
+        if (site == 0) continue;
+        words[f] = 0;
+        return fail(RT_ERR_CUDA, std::string(WAIT_FAMILIES[f].what) + " gave up a bounded wait (site " + std::to_string(site) + "): " + WAIT_FAMILIES[f].left);
+    }
     return RT_OK;
 }
 
@@ -493,11 +526,32 @@ rt_status rt_upload(rt_device *dev, rt_buffer *dst, uint64_t dst_off, const void
     return RT_OK;
 }
 
+// A small result for pageable memory (logits, a hidden row) goes through a page-locked area of the device's own: the
+// driver's path for pageable destinations costs more than the copy does up to a few hundred KB.
+static constexpr uint64_t STAGE_BYTES = 256u << 10;
+static bool is_page_locked(const void *host) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
 rt_status rt_download(rt_device *dev, const rt_buffer *src, uint64_t src_off, void *host, uint64_t n, int32_t sync) {
     if (!dev || !src || (!host && n)) return fail(RT_ERR_ARG, "rt_download: null argument");
     if (src_off > src->size || n > src->size - src_off) return fail(RT_ERR_ARG, "rt_download: range exceeds the buffer");
     CUDA_TRY(cudaSetDevice(dev->ordinal));
-    if (n) CUDA_TRY(cudaMemcpyAsync(host, (const char *)src->ptr + src_off, n, cudaMemcpyDeviceToHost, dev->stream));
+    const void *const from = (const char *)src->ptr + src_off;
+    if (sync && n && n <= STAGE_BYTES && !is_page_locked(host)) {
+        std::lock_guard<std::mutex> lk(dev->stage_mu);
+        if (!dev->stage) CUDA_TRY(cudaMallocHost(&dev->stage, STAGE_BYTES));
+        CUDA_TRY(cudaMemcpyAsync(dev->stage, from, n, cudaMemcpyDeviceToHost, dev->stream));
+        CUDA_TRY(cudaStreamSynchronize(dev->stream));
+        memcpy(host, dev->stage, n);
+        return RT_OK;
+    }
+    if (n) CUDA_TRY(cudaMemcpyAsync(host, from, n, cudaMemcpyDeviceToHost, dev->stream));
     if (sync) CUDA_TRY(cudaStreamSynchronize(dev->stream));
     return RT_OK;
 }
@@ -931,6 +985,55 @@ rt_status rt_matmul_launch(rt_plan *plan, const void *lhs, const void *rhs, cons
 rt_status rt_matmul_launch_ex(rt_plan *plan, const void *lhs, const void *rhs, const void *bias, void *out, void *stream,
                               const rt_launch_opts *opts) {
     return launch_node(plan, lhs, rhs, bias, out, stream, opts, nullptr);
+}
+
+uint64_t rt_routing_stamp(void) {
+    static std::mutex mu;
+    static std::unordered_map<std::string, uint64_t> seen;
+    const std::string now = routing_switches();
+    std::lock_guard<std::mutex> lk(mu);
+    return seen.emplace(now, seen.size()).first->second;
+}
+
+rt_status rt_graph_resolve(rt_device *dev, const uint64_t *nodes, int32_t n, uint64_t *outs, int32_t *n_done) {
+    if (n_done) *n_done = 0;
+    if (!dev || n < 0 || (n > 0 && (!nodes || !outs)) || !n_done) return fail(RT_ERR_ARG, "rt_graph_resolve: bad argument");
+    for (int32_t i = 0; i < n; i++) {
+        const uint64_t *d = nodes + (size_t)i * 5;
+        rt_plan *plan = reinterpret_cast<rt_plan *>(d[0]);
+        if (!plan || plan->dev != dev) return fail(RT_ERR_ARG, "rt_graph_resolve: node without a plan of this device");
+        const void *operand[3];
+        for (int k = 0; k < 3; k++) {
+            const uint64_t v = d[1 + k];
+            if (v & 1) {
+                if (v >> 1 >= (uint64_t)i) return fail(RT_ERR_ARG, "rt_graph_resolve: a node reads a later node's output");
+                operand[k] = reinterpret_cast<const void *>(outs[(v >> 1) * 3 + 1]);
+            } else {
+                operand[k] = reinterpret_cast<const void *>(v);
+            }
+        }
+        rt_segment seg[2];
+        int nseg = 0;
+        uint64_t bytes = 0;
+        Status st = dtype_segments(plan->spec.out_dt, (uint64_t)numel(plan->spec.out_shape), seg, &nseg);
+        if (!st.ok()) return fail(st);
+        for (int k = 0; k < nseg; k++) bytes += seg[k].size;
+        rt_buffer *buf = nullptr;
+        rt_status rs = rt_buffer_alloc(dev, bytes, &buf);
+        if (rs != RT_OK) return rs;
+        rt_launch_opts opts = {};
+        opts.flags = (uint32_t)d[4];
+        rs = launch_node(plan, operand[0], operand[1], operand[2], buf->ptr, nullptr, &opts, nullptr);
+        if (rs != RT_OK) {
+            rt_buffer_free(buf);
+            return rs;
+        }
+        outs[(size_t)i * 3] = reinterpret_cast<uint64_t>(buf);
+        outs[(size_t)i * 3 + 1] = reinterpret_cast<uint64_t>(buf->ptr);
+        outs[(size_t)i * 3 + 2] = buf->size;
+        *n_done = i + 1;
+    }
+    return RT_OK;
 }
 
 } // extern "C"

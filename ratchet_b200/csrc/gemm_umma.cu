@@ -16,9 +16,9 @@
 //   warps 2-9   epilogue: tcgen05.ld of one of two accumulator buffers (so the next tile's MMAs
 //               overlap), the reference's epilogue chain, stores staged through shared memory so
 //               that every store instruction writes whole 128-byte lines
-// Every wait is bounded (about two seconds of SM cycles); on expiry the kernel records the wait site in a device
-// flag, all roles leave their loops, tensor memory is freed and the kernel returns.  The host
-// reads the flag at the next rt_device_sync.
+// Every wait is bounded (about two seconds of SM cycles); on expiry the kernel reports the wait site to a host word
+// (wait_error.cuh), all roles leave their loops, tensor memory is freed and the kernel returns.  The host
+// reads the word at the next rt_device_sync.
 #include <cuda.h>
 
 #include <algorithm>
@@ -30,10 +30,9 @@
 
 #include "common.cuh"
 #include "kernels.hpp"
+#include "wait_error.cuh"
 
 namespace rt {
-
-__device__ int g_umma_error = 0;
 
 namespace {
 
@@ -118,7 +117,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (*abort_flag) return false;
         if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
             *abort_flag = 1;
-            atomicCAS(&g_umma_error, 0, site);
+            report_wait_error(site);
             return false;
         }
     }
@@ -1025,15 +1024,6 @@ cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dty
     return cudaErrorInvalidValue;
 }
 
-// Reads and clears the wait-expiry flag (0 = no kernel gave up a wait).
-cudaError_t umma_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_umma_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_umma_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t umma_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

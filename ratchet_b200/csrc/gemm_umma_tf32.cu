@@ -39,8 +39,6 @@
 
 namespace rt {
 
-__device__ int g_umma_tf32_error = 0;
-
 namespace {
 
 using namespace umma_gemv; // smem_u32, mbarrier helpers, fences, encode_tiled_fn
@@ -86,7 +84,7 @@ __device__ __forceinline__ void tmem_ld8_f32(uint32_t taddr, uint32_t (&v)[8]) {
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site) {
-    return mbar_wait_flag(bar, parity, abort_flag, site, &g_umma_tf32_error);
+    return mbar_wait_flag(bar, parity, abort_flag, site);
 }
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar) {
@@ -485,14 +483,6 @@ cudaError_t launch_gemm_umma_tf32x3(const void *P, const void *Q, void *out, int
     }
 }
 
-cudaError_t umma_tf32_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_umma_tf32_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_umma_tf32_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t umma_tf32_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

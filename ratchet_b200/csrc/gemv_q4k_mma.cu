@@ -30,12 +30,11 @@
 #include "common.cuh"
 #include "decode.cuh"
 #include "kernels.hpp"
+#include "wait_error.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace rt {
-
-__device__ int g_gemv_q4k_error = 0;
 
 namespace {
 
@@ -223,7 +222,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == WARPS_WALK ? 1 : 0) q4k_g
             while (!mbar_try_wait(bar, parity)) {
                 if ((unsigned long long)clock64() - t0 > WAIT_LIMIT_CYCLES) {
                     ok = false;
-                    atomicCAS(&g_gemv_q4k_error, 0, 1);
+                    report_wait_error(1);
                     break;
                 }
             }
@@ -455,14 +454,6 @@ cudaError_t launch_q4k_gemv(const MatmulParams &p, int nv, int config, bool lhs_
                    : launch_g<2>(p, nv, split, gpc, nbuf, lhs_constant, stream);
 }
 
-cudaError_t gemv_q4k_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_gemv_q4k_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_gemv_q4k_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t gemv_q4k_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

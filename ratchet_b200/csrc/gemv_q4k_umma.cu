@@ -40,8 +40,6 @@ namespace cg = cooperative_groups;
 
 namespace rt {
 
-__device__ int g_gemv_q4k_umma_error = 0;
-
 namespace {
 
 using namespace umma_gemv;
@@ -88,7 +86,7 @@ struct Q4kUmmaParams {
 };
 
 __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site) {
-    return mbar_wait_flag(bar, parity, abort_flag, site, &g_gemv_q4k_umma_error);
+    return mbar_wait_flag(bar, parity, abort_flag, site);
 }
 
 // Bounded wait.  The waiting warp sleeps between tries: a spinning warp's tries go through the same shared-memory
@@ -106,7 +104,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (*abort_flag) return false;
         if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
             *abort_flag = 1;
-            atomicCAS(&g_gemv_q4k_umma_error, 0, site);
+            report_wait_error(site);
             return false;
         }
     }
@@ -464,7 +462,7 @@ q4k_gemv_umma_kernel(const __grid_constant__ CUtensorMap map_w, const Q4kUmmaPar
                              : "=r"(done) : "r"(bar_red) : "memory");
                 if (!done && wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
                     *abort_flag = 1;
-                    atomicCAS(&g_gemv_q4k_umma_error, 0, 9);
+                    report_wait_error(9);
                     break;
                 }
             }
@@ -611,14 +609,6 @@ cudaError_t launch_q4k_gemv_umma(const MatmulParams &p, int nv, const Q4kUmmaCon
     return cudaLaunchKernelEx(&lc, kernel, map_w, up);
 }
 
-cudaError_t gemv_q4k_umma_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_gemv_q4k_umma_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_gemv_q4k_umma_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t gemv_q4k_umma_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

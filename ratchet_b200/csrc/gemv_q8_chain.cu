@@ -48,8 +48,6 @@
 
 namespace rt {
 
-__device__ int g_gemv_chain_error = 0;
-
 namespace {
 
 using namespace umma_gemv;
@@ -119,7 +117,7 @@ struct ChainParams {
 };
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site) {
-    return mbar_wait_flag(bar, parity, abort_flag, site, &g_gemv_chain_error);
+    return mbar_wait_flag(bar, parity, abort_flag, site);
 }
 
 __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainParams cp) {
@@ -376,7 +374,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
                                 if (*abort_flag) break;
                                 if (wait_clock() - t0 > cp.poll_limit) {
                                     *abort_flag = 1;
-                                    atomicCAS(&g_gemv_chain_error, 0, 8);
+                                    report_wait_error(8);
                                     break;
                                 }
                             }
@@ -531,7 +529,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
                                 if (*abort_flag) break;
                                 if (wait_clock() - t0 > cp.poll_limit) {
                                     *abort_flag = 1;
-                                    atomicCAS(&g_gemv_chain_error, 0, 7);
+                                    report_wait_error(7);
                                     break;
                                 }
                             }
@@ -550,7 +548,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
                                     if (*abort_flag) break;
                                     if (wait_clock() - t0 > cp.poll_limit) {
                                         *abort_flag = 1;
-                                        atomicCAS(&g_gemv_chain_error, 0, 7);
+                                        report_wait_error(7);
                                         break;
                                     }
                                 }
@@ -824,14 +822,6 @@ cudaError_t gemv_chain_launch(GemvChain *c, cudaStream_t stream) {
     return cudaLaunchKernelEx(&lc, q8_gemv_chain_kernel, c->cp);
 }
 
-cudaError_t gemv_chain_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_gemv_chain_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_gemv_chain_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t gemv_chain_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

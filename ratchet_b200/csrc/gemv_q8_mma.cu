@@ -27,12 +27,11 @@
 
 #include "common.cuh"
 #include "kernels.hpp"
+#include "wait_error.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace rt {
-
-__device__ int g_gemv_error = 0;
 
 namespace {
 
@@ -158,7 +157,7 @@ __global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p
         while (!mbar_try_wait(bar_addr, 0)) {
             if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
                 ok = false;
-                atomicCAS(&g_gemv_error, 0, 1);
+                report_wait_error(1);
                 break;
             }
         }
@@ -323,14 +322,6 @@ cudaError_t launch_q8_gemv_mma(const MatmulParams &p, bool f32_scales, int nv, i
                       : launch_scale<__half>(p, nv, split, lhs_constant, stream);
 }
 
-cudaError_t gemv_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_gemv_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_gemv_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t gemv_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

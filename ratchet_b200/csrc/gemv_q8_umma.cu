@@ -40,8 +40,6 @@ namespace cg = cooperative_groups;
 
 namespace rt {
 
-__device__ int g_gemv_umma_error = 0;
-
 namespace {
 
 constexpr int THREADS = 288;          // warp 0: TMA producer, warps 1, 6, 7, 8: MMA issuers, warps 2-5: digits + epilogue
@@ -67,7 +65,7 @@ struct UmmaGemvParams {
 using namespace umma_gemv;
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site) {
-    return mbar_wait_flag(bar, parity, abort_flag, site, &g_gemv_umma_error);
+    return mbar_wait_flag(bar, parity, abort_flag, site);
 }
 
 // Shared-memory map (all offsets from a 1024-byte aligned base):
@@ -291,7 +289,7 @@ q8_gemv_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                              : "=r"(done) : "r"(bar_red) : "memory");
                 if (!done && wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
                     *abort_flag = 1;
-                    atomicCAS(&g_gemv_umma_error, 0, 7);
+                    report_wait_error(7);
                     break;
                 }
             }
@@ -410,14 +408,6 @@ cudaError_t launch_q8_gemv_umma(const MatmulParams &p, const GemvUmmaConfig &cfg
     return cudaLaunchKernelEx(&lc, q8_gemv_umma_kernel, map_w, map_s, up);
 }
 
-cudaError_t gemv_umma_take_error(int *site, cudaStream_t stream) {
-    int zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbolAsync(site, g_gemv_umma_error, sizeof(int), 0, cudaMemcpyDeviceToHost, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return e;
-    if (*site != 0) e = cudaMemcpyToSymbolAsync(g_gemv_umma_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, stream);
-    return e;
-}
+cudaError_t gemv_umma_bind_wait_error(int *word) { return bind_wait_error(word); }
 
 } // namespace rt

@@ -58,7 +58,7 @@ cudaError_t launch_rowvec_mat(const MatmulParams &p, rt_dtype dt, int chunks, fl
 // kernel may request them before it waits for its stream predecessor.
 int q8_gemv_mma_pick_split(int M, int K, int sm_count, int scale_size);
 cudaError_t launch_q8_gemv_mma(const MatmulParams &p, bool f32_scales, int nv, int split, bool lhs_constant, cudaStream_t stream);
-cudaError_t gemv_take_error(int *site, cudaStream_t stream);
+cudaError_t gemv_bind_wait_error(int *word);
 
 // Q8_0H x f16 GEMV on tcgen05 kind::i8 (one activation vector, stacks == 1, K % 256 == 0).
 struct GemvUmmaConfig {
@@ -67,7 +67,7 @@ struct GemvUmmaConfig {
 };
 bool q8_gemv_umma_config(int M, int K, int sm_count, GemvUmmaConfig *cfg);
 cudaError_t launch_q8_gemv_umma(const MatmulParams &p, const GemvUmmaConfig &cfg, bool lhs_constant, cudaStream_t stream);
-cudaError_t gemv_umma_take_error(int *site, cudaStream_t stream);
+cudaError_t gemv_umma_bind_wait_error(int *word);
 
 // A list of such GEMVs (constant weights, node l+1 may read what node l wrote) as one persistent
 // cooperative kernel with grid barriers between the nodes.  gemv_chain_create returns cudaSuccess
@@ -77,12 +77,12 @@ cudaError_t gemv_chain_create(const std::vector<MatmulParams> &nodes, int device
 cudaError_t gemv_chain_launch(GemvChain *chain, cudaStream_t stream);
 void gemv_chain_destroy(GemvChain *chain);
 const char *gemv_chain_name(const GemvChain *chain);
-cudaError_t gemv_chain_take_error(int *site, cudaStream_t stream);
+cudaError_t gemv_chain_bind_wait_error(int *word);
 
 // Q4_K x f16 GEMV / skinny GEMM on warp MMAs.  nv = columns of op(rhs), 1..16 (rhs stored [nv][K]).
 int q4k_gemv_pick_split(int M, int K, int nv, int stacks, int sm_count); // split | groups per CTA << 8 | weight buffers << 16, or 0
 cudaError_t launch_q4k_gemv(const MatmulParams &p, int nv, int config, bool lhs_constant, cudaStream_t stream);
-cudaError_t gemv_q4k_take_error(int *site, cudaStream_t stream);
+cudaError_t gemv_q4k_bind_wait_error(int *word);
 
 // Q4_K GEMV / skinny GEMM through tensor memory (gemv_q4k_umma.cu): raw super-blocks by TMA, nibbles to int8 codes
 // in shared memory, tcgen05.mma kind::i8 against block-floating digits of the activations.
@@ -92,7 +92,7 @@ struct Q4kUmmaConfig {
 };
 bool q4k_gemv_umma_config(int M, int K, int nv, int sm_count, Q4kUmmaConfig *cfg);
 cudaError_t launch_q4k_gemv_umma(const MatmulParams &p, int nv, const Q4kUmmaConfig &cfg, bool lhs_constant, cudaStream_t stream);
-cudaError_t gemv_q4k_umma_take_error(int *site, cudaStream_t stream);
+cudaError_t gemv_q4k_umma_bind_wait_error(int *word);
 
 // Dense f32 GEMM on the tensor cores, three TF32 MMAs per product (f32-class accuracy): D[R][S] = P[R][K] . Q[S][K]^T.
 bool umma_tf32_supported(long long K);
@@ -101,7 +101,7 @@ bool umma_tf32_presplit_pays(int S, int bn);
 cudaError_t launch_gemm_umma_tf32x3(const void *P, const void *Q, void *out, int R, int S, int K, int stacks, int p_stack, int q_stack,
                                     const void *bias, int bias_dt, int bias_mode, int epilogue, int bn, void *p_split, int sm_count,
                                     cudaStream_t stream);
-cudaError_t umma_tf32_take_error(int *site, cudaStream_t stream);
+cudaError_t umma_tf32_bind_wait_error(int *word);
 
 // Tensor-core GEMM (tcgen05): D[R][S] = P[R][K] . Q[S][K]^T, 16-bit K-major operands, bias along S.
 // Several destinations for one result: see UmmaParams in gemm_umma.cu.  p_scale [p_stack][R] / q_scale [q_stack][S]:
@@ -119,8 +119,8 @@ cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dty
                              int R, int S, int K, int stacks, int p_stack, int q_stack, const void *bias, int bias_dt,
                              int bias_mode, int epilogue, int bn, int sm_count, cudaStream_t stream,
                              const UmmaScatter *scatter = nullptr, const float *p_scale = nullptr, const float *q_scale = nullptr);
-// Reads and clears the device flag a kernel sets when one of its bounded waits expires.
-cudaError_t umma_take_error(int *site, cudaStream_t stream);
+// (every *_bind_wait_error: the host word in which that file's kernels report a bounded wait that expired, for the current device)
+cudaError_t umma_bind_wait_error(int *word);
 
 // Block-format tensor -> f32 / f16 values.
 cudaError_t launch_dequant(rt_dtype dt, long long numel, const void *src, const void *scales, void *dst, rt_dtype out_dt,

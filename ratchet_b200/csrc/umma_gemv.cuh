@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "wait_error.cuh"
+
 namespace rt {
 namespace umma_gemv {
 
@@ -44,9 +46,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up after WAIT_LIMIT_CYCLES, or as soon as the CTA's abort flag is up; the first
-// site that gives up is recorded in *error_word (a __device__ int the host reads at its next sync).
-__device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site, int *error_word) {
+// Bounded wait: gives up after WAIT_LIMIT_CYCLES, or as soon as the CTA's abort flag is up; the
+// site that gives up is reported to the host, which looks at its next sync.
+__device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site) {
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = wait_clock();
     while (true) {
@@ -56,7 +58,7 @@ __device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, vo
         if (*abort_flag) return false;
         if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
             *abort_flag = 1;
-            atomicCAS(error_word, 0, site);
+            report_wait_error(site);
             return false;
         }
     }

@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import math
 import os
 from ctypes import byref, c_int32, c_uint64, c_void_p
 from typing import Optional, Sequence
@@ -64,6 +65,8 @@ class DType(enum.IntEnum):
                 DType.I32: np.int32, DType.U32: np.uint32}.get(self, np.uint8)
 
 
+_DTYPES = {int(d): d for d in DType}
+
 _NP_TO_DT = {np.dtype(np.float32): DType.F32, np.dtype(np.float16): DType.F16,
              np.dtype(np.int32): DType.I32, np.dtype(np.uint32): DType.U32}
 
@@ -79,11 +82,6 @@ def f32_to_bf16_bits(x: np.ndarray) -> np.ndarray:
 
 def bf16_bits_to_f32(bits: np.ndarray) -> np.ndarray:
     return (np.ascontiguousarray(bits, dtype=np.uint16).astype(np.uint32) << 16).view(np.float32)
-
-
-# environment switches that change which kernel a plan takes (the library's cache key holds them too)
-_ROUTING_SWITCHES = ("RT_FORCE_KERNEL", "RT_GEMV_UMMA", "RT_Q4K_UMMA", "RT_GEMM_PAIR", "RT_GEMM_PAIR_MIN", "RT_TF32_BN",
-                     "RT_TF32_PRESPLIT", "RT_Q4K_WALK_FROM", "RT_KEEP_WEIGHTS")
 
 
 class DeviceRequest(enum.Enum):
@@ -139,7 +137,7 @@ class Device:
         # The library keeps the cache (keyed by the description and by the routing switches of the environment); this
         # memo only saves the two calls per node on the lazy path.  The hold rt_matmul_plan takes goes straight back:
         # the device's own keeps the plan alive as long as the device lives.
-        key = (bytes(desc), tuple(os.environ.get(n) for n in _ROUTING_SWITCHES))
+        key = (bytes(desc), _lib.load().rt_routing_stamp())
         h = self._plans.get(key)
         if h is None:
             h = c_void_p()
@@ -199,6 +197,45 @@ class GpuBuffer:
                 self._h = None
         except Exception:
             pass
+
+
+class _NodeForm:
+    """What a Matmul node is apart from its data: its description, what the library's rules say of it, and its plans.
+    Pure functions of dtypes, shapes and flags, so equal nodes share one (a decode step asks for the same few forms token
+    after token; working one out again costs more than launching its kernel)."""
+
+    __slots__ = ("desc", "spec", "out_shape", "out_dt", "_plans")
+    _known: dict = {}
+    LIMIT = 4096  # forms kept; a program with more distinct shapes starts over
+
+    def __init__(self, desc: "_lib.rt_matmul_desc"):
+        self.desc = desc
+        # Matmul::new guards, check_shapes, check_dtypes: all evaluated by the library
+        self.spec = _lib.rt_gemm_spec()
+        check(_lib.load().rt_matmul_spec(byref(desc), byref(self.spec)))
+        self.out_shape = self.spec.out_shape.tolist()
+        self.out_dt = _DTYPES[self.spec.out_dt]
+        self._plans = {}
+
+    @classmethod
+    def of(cls, op: "Matmul") -> "_NodeForm":
+        lhs, rhs, bias = op.lhs, op.rhs, op.bias
+        key = (lhs.dt._value_, tuple(lhs.shape), rhs.dt._value_, tuple(rhs.shape),
+               None if bias is None else (bias.dt._value_, tuple(bias.shape)), op.trans_lhs, op.trans_rhs, op.trans_out, op.epilogue)
+        form = cls._known.get(key)
+        if form is None:
+            form = cls(op._desc())
+            if len(cls._known) >= cls.LIMIT:
+                cls._known.clear()
+            cls._known[key] = form
+        return form
+
+    def plan(self, device: Device, stamp: int) -> int:
+        key = (device._h.value, stamp)
+        h = self._plans.get(key)
+        if h is None:
+            h = self._plans[key] = device.plan_for(self.desc).value
+        return h
 
 
 class Executable:
@@ -285,10 +322,15 @@ class Matmul:
         self.lhs, self.rhs, self.bias = lhs, rhs, bias
         self.trans_lhs, self.trans_rhs, self.trans_out = bool(trans_lhs), bool(trans_rhs), bool(trans_out)
         self.epilogue = int(epilogue)
-        self.desc = self._desc()
-        # Matmul::new guards, check_shapes, check_dtypes: all evaluated by the library
-        self.spec = _lib.rt_gemm_spec()
-        check(_lib.load().rt_matmul_spec(byref(self.desc), byref(self.spec)))
+        self._form = _NodeForm.of(self)
+
+    @property
+    def desc(self) -> "_lib.rt_matmul_desc":
+        return _lib.rt_matmul_desc.from_buffer_copy(self._form.desc)
+
+    @property
+    def spec(self) -> "_lib.rt_gemm_spec":
+        return _lib.rt_gemm_spec.from_buffer_copy(self._form.spec)
 
     def _desc(self) -> "_lib.rt_matmul_desc":
         d = _lib.rt_matmul_desc()
@@ -367,7 +409,7 @@ class Tensor:
 
     # ------------------------------------------------------------------ properties
     def numel(self) -> int:
-        return int(np.prod(self.shape)) if self.shape else 1
+        return math.prod(self.shape)
 
     def rank(self) -> int:
         return len(self.shape)
@@ -389,7 +431,9 @@ class Tensor:
              epilogue: int = _lib.RT_EPILOGUE_NONE) -> "Tensor":
         """Tensor::gemm (tensor.rs:388-400): self is the lhs."""
         op = Matmul(self, rhs, bias, trans_lhs, trans_rhs, trans_out, epilogue)
-        return Tensor(op.spec.out_shape.tolist(), DType(op.spec.out_dt), rhs.device, None, op)
+        t = Tensor.__new__(Tensor)
+        t.shape, t.dt, t.device, t.storage, t.op = op._form.out_shape.copy(), op._form.out_dt, rhs.device, None, op
+        return t
 
     def matmul(self, rhs: "Tensor", trans_lhs: bool = False, trans_rhs: bool = False) -> "Tensor":
         """Tensor::matmul (tensor.rs:381-386)."""
@@ -398,44 +442,58 @@ class Tensor:
     # ------------------------------------------------------------------ execution
     def execution_order(self):
         """Post-order over the op graph (tensor.rs:667-711)."""
-        order, seen, stack = [], set(), [(self, False)]
+        order, seen, stack = [], set(), [self]
         while stack:
-            t, done = stack.pop()
-            if done:
-                order.append(t)
+            t = stack.pop()
+            if t is None:  # everything below the next tensor is in the order
+                order.append(stack.pop())
                 continue
             if id(t) in seen:
                 continue
             seen.add(id(t))
-            stack.append((t, True))
-            if t.op is not None and not t.resolved():
-                for s in reversed(t.op.srcs()):
-                    stack.append((s, False))
+            op = t.op
+            if op is None or t.storage is not None:
+                order.append(t)
+                continue
+            stack += (t, None)
+            if op.bias is not None:
+                stack.append(op.bias)
+            stack += (op.rhs, op.lhs)
         return order
 
     def resolve(self, sync: bool = True) -> "Tensor":
         """Tensor::resolve (tensor.rs:738-787): plan + dispatch every unresolved node, then wait."""
         device = self.device.try_gpu()
         lib = _lib.load()
-        todo = [t for t in self.execution_order() if not t.resolved()]
-        for t in todo:
-            if t.op is None:
-                raise RatchetError(_lib.RT_ERR_ARG, "RT_ERR_ARG", "unresolved tensor without an op")
-            for s in t.op.srcs():
-                if s.resolved() and (not isinstance(s.storage, GpuBuffer) or s.device is not device):
-                    raise RatchetError(_lib.RT_ERR_ARG, "RT_ERR_ARG",
-                                       f"TensorError: operand on {s.device}, expected {device}")
-        for i, t in enumerate(todo):
-            op = t.op
-            plan = device.plan_for(op.desc)
-            out = GpuBuffer(device, t.nbytes())
-            opts = _lib.rt_launch_opts()
-            # a leaf lhs is a constant of the graph (uploaded weights): nothing in flight writes it
-            if op.lhs.op is None:
-                opts.flags = _lib.RT_LAUNCH_LHS_CONSTANT
-            check(lib.rt_matmul_launch_ex(plan, op.lhs.ptr, op.rhs.ptr, op.bias.ptr if op.bias is not None else None,
-                                          out.ptr, None, byref(opts)))
-            t.storage = out
+        todo = [t for t in self.execution_order() if t.storage is None]
+        if todo:
+            position = {id(t): i for i, t in enumerate(todo)}
+            stamp = lib.rt_routing_stamp()
+            words = []  # per node: plan, lhs, rhs, bias, flags (rt_graph_resolve)
+            for t in todo:
+                op = t.op
+                if op is None:
+                    raise RatchetError(_lib.RT_ERR_ARG, "RT_ERR_ARG", "unresolved tensor without an op")
+                words.append(op._form.plan(device, stamp))
+                for s in (op.lhs, op.rhs, op.bias):
+                    if s is None:
+                        words.append(0)
+                    elif s.storage is None:
+                        words.append(2 * position[id(s)] + 1)
+                    elif isinstance(s.storage, GpuBuffer) and s.device is device:
+                        words.append(s.storage.ptr)
+                    else:
+                        raise RatchetError(_lib.RT_ERR_ARG, "RT_ERR_ARG", f"TensorError: operand on {s.device}, expected {device}")
+                # a leaf lhs is a constant of the graph (uploaded weights): nothing in flight writes it
+                words.append(_lib.RT_LAUNCH_LHS_CONSTANT if op.lhs.op is None else 0)
+            n = len(todo)
+            outs, done = (c_uint64 * (3 * n))(), c_int32()
+            status = lib.rt_graph_resolve(device._h, (c_uint64 * len(words))(*words), n, outs, byref(done))
+            for i, t in zip(range(done.value), todo):
+                b = GpuBuffer.__new__(GpuBuffer)
+                b.device, b._h, b.ptr, b.size = device, outs[3 * i], outs[3 * i + 1], outs[3 * i + 2]
+                t.storage = b
+            check(status)
         if sync:
             device.sync()
         return self
@@ -450,14 +508,14 @@ class Tensor:
         if device.is_gpu() and not self.device.is_gpu():
             buf = GpuBuffer(device, self.nbytes())
             raw = self.storage
-            check(lib.rt_upload(device._h, buf._h, 0, raw.ctypes.data_as(c_void_p), raw.size, 1))
+            check(lib.rt_upload(device._h, buf._h, 0, raw.ctypes.data, raw.size, 1))
             return Tensor(self.shape, self.dt, device, buf)
         if not device.is_gpu() and self.device.is_gpu():
             n = self.nbytes()
             raw = out.view(np.uint8).reshape(-1) if out is not None else np.empty(n, dtype=np.uint8)
             if raw.size < n:
                 raise RatchetError(_lib.RT_ERR_ARG, "RT_ERR_ARG", "output array too small")
-            check(lib.rt_download(self.device._h, self.storage._h, 0, raw.ctypes.data_as(c_void_p), n, 1))
+            check(lib.rt_download(self.device._h, self.storage._h, 0, raw.ctypes.data, n, 1))
             return Tensor(self.shape, self.dt, Device.CPU, raw[:n])
         raise RatchetError(_lib.RT_ERR_UNSUPPORTED, "RT_ERR_UNSUPPORTED", "GPU to GPU moves are not part of this path")
 
@@ -469,7 +527,7 @@ class Tensor:
         raw = np.ascontiguousarray(data).view(np.uint8).reshape(-1)
         if raw.size != self.nbytes():
             raise RatchetError(_lib.RT_ERR_ARG, "RT_ERR_ARG", f"write: {raw.size} bytes for a tensor of {self.nbytes()}")
-        check(_lib.load().rt_upload(self.device._h, self.storage._h, 0, raw.ctypes.data_as(c_void_p), raw.size, 0))
+        check(_lib.load().rt_upload(self.device._h, self.storage._h, 0, raw.ctypes.data, raw.size, 0))
         return self
 
     # ------------------------------------------------------------------ host views
