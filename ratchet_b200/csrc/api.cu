@@ -87,7 +87,7 @@ struct rt_plan {
     uint64_t lhs_scale_offset = 0;
     // tensor-core GEMM: operand roles, tile width, and the scratch that holds dequantised weights
     bool lhs_is_q = false; // the lhs is the kernel's Q operand (trans_out), else its P operand
-    int R = 0, S = 0, u_stacks = 1, p_stack = 1, q_stack = 1, bn = 128;
+    int R = 0, S = 0, u_stacks = 1, p_stack = 1, q_stack = 1, bn = 128, ksplit = 1;
     bool tf32x3 = false;   // dense f32 on the tensor cores: three TF32 MMAs per product
     bool rhs_transpose = false; // rhs is stored [K][N]: transposed into act_scratch ahead of the GEMM
     int k_pad = 0;              // with rhs_transpose, 16-bit: K rounded up to a multiple of 8 when it is not one
@@ -155,7 +155,7 @@ static cudaError_t bind_wait_words(int ordinal) {
 }
 
 // The environment switches that change which kernel a plan takes.
-static const char *const ROUTING_SWITCHES[] = {"RT_FORCE_KERNEL", "RT_GEMV_UMMA", "RT_Q4K_UMMA", "RT_GEMM_PAIR", "RT_GEMM_PAIR_MIN",
+static const char *const ROUTING_SWITCHES[] = {"RT_FORCE_KERNEL", "RT_GEMV_UMMA", "RT_Q4K_UMMA", "RT_GEMM_PAIR", "RT_GEMM_PAIR_MIN", "RT_GEMM_KSPLIT",
                                                "RT_TF32_BN", "RT_TF32_PRESPLIT", "RT_Q4K_WALK_FROM", "RT_KEEP_WEIGHTS"};
 static std::string routing_switches() {
     std::string k;
@@ -795,12 +795,13 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
         pl->p_stack = s.trans_out ? rhs_st : lhs_st;
         pl->q_stack = s.trans_out ? lhs_st : rhs_st;
         pl->tf32x3 = desc->rhs_dt == RT_F32;
-        pl->bn = pl->tf32x3 ? umma_tf32_pick_bn(pl->R, pl->S, pl->u_stacks, dev->sm_count)
-                            : umma_pick_bn(pl->R, pl->S, pl->u_stacks, dev->sm_count);
+        if (pl->tf32x3) pl->bn = umma_tf32_pick_bn(pl->R, pl->S, pl->u_stacks, dev->sm_count);
+        else if (cudaSetDevice(dev->ordinal) == cudaSuccess)
+            umma_pick_tile(pl->R, pl->S, s.K, pl->u_stacks, s.epilogue == RT_EPILOGUE_SILU_MUL, dev->sm_count, &pl->bn, &pl->ksplit);
         // problems that fill most of a wave of SM pairs with 256 x 256 tiles: two CTAs per tile (tcgen05 cta_group::2)
         if (!pl->tf32x3 && s.epilogue != RT_EPILOGUE_SILU_MUL && gemm_pair_enabled() && dev->sm_count >= 2 &&
             (long long)((pl->R + 255) / 256) * ((pl->S + 255) / 256) * pl->u_stacks >= gemm_pair_min_tiles(dev->sm_count))
-            pl->bn = UMMA_BN_PAIR;
+            pl->bn = UMMA_BN_PAIR, pl->ksplit = 1;
         pl->launches = 1;
         if (!s.trans_rhs) {
             pl->rhs_transpose = true;
@@ -879,7 +880,8 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
             }
         }
         pl->name = std::string(pl->tf32x3 ? "gemm_umma_tf32x3_" : "gemm_umma_") + dtype_name(desc->lhs_dt) + "_" + dtype_name(desc->rhs_dt) +
-                   (pl->bn == UMMA_BN_PAIR ? std::string("_pair256x256") : "_bn" + std::to_string(pl->bn)) + (pl->scratch && !pl->k_pad ? (pl->tf32x3 ? "_presplit" : "_dequant_prepass") : "") + (pl->wdq ? "_dequant_prepass" : "") +
+                   (pl->bn == UMMA_BN_PAIR ? std::string("_pair256x256") : "_bn" + std::to_string(pl->bn)) +
+                   (pl->ksplit > 1 ? "_ksplit" + std::to_string(pl->ksplit) : std::string()) + (pl->scratch && !pl->k_pad ? (pl->tf32x3 ? "_presplit" : "_dequant_prepass") : "") + (pl->wdq ? "_dequant_prepass" : "") +
                    (pl->rhs_transpose ? "_rhs_transposed" : "") + (pl->k_pad ? "_kpad" + std::to_string(pl->k_pad) : "");
     } else if (s.N == 1 && !s.trans_lhs) {
         pl->kernel = PK_GEMV_SIMT;
@@ -1193,7 +1195,7 @@ static rt_status launch_node(rt_plan *plan, const void *lhs, const void *rhs, co
         e = launch_gemm_umma(P, p_dt, Q, q_dt, out, s.out_dt, plan->R, plan->S, k_eff, plan->u_stacks, plan->p_stack,
                              plan->q_stack, p.bias, p.bias_dt, s.has_bias ? BIAS_PER_N : BIAS_NONE, p.epilogue, plan->bn,
                              plan->dev->sm_count, st, scatter ? &sc : nullptr, plan->lhs_is_q ? x_scale : nullptr,
-                             plan->lhs_is_q ? nullptr : x_scale);
+                             plan->lhs_is_q ? nullptr : x_scale, plan->ksplit);
         break;
     }
     }

@@ -22,6 +22,8 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <climits>
+#include <cstdio>
 #include <unordered_map>
 #include <string>
 #include <mutex>
@@ -802,6 +804,8 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_co
     }
 }
 
+#include "gemm_umma_ksplit.cuh"
+
 // ------------------------------------------------------------------------------------------ host side
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -901,6 +905,72 @@ cudaError_t launch_bn(const CUtensorMap &mp, const CUtensorMap &mq, UmmaParams p
     return launch_pdl(kernel, dim3(grid), dim3(NUM_THREADS), C::SMEM_BYTES, stream, mp, mq, prm);
 }
 
+template <int BN, typename OutT>
+cudaError_t launch_ksplit(const CUtensorMap &mp, const CUtensorMap &mq, UmmaParams prm, int ksplit, cudaStream_t stream) {
+    using C = KsCfg<BN>;
+    if (ksplit < 2 || ksplit > UMMA_KSPLIT_MAX || ksplit > (prm.K + BK - 1) / BK) return cudaErrorInvalidValue;
+    static SmemAttr smem_attr[4];
+    const bool wide = ksplit > 4;
+    auto kernel = prm.pair ? (wide ? gemm_umma_ksplit_kernel<BN, OutT, true, 8> : gemm_umma_ksplit_kernel<BN, OutT, true, 4>)
+                           : (wide ? gemm_umma_ksplit_kernel<BN, OutT, false, 8> : gemm_umma_ksplit_kernel<BN, OutT, false, 4>);
+    cudaError_t e = smem_attr[(prm.pair ? 2 : 0) + (wide ? 1 : 0)].ensure(kernel, C::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    prm.tiles_r = (prm.R + BM - 1) / BM;
+    prm.group_r = prm.tiles_r;
+    prm.tiles_s = prm.pair ? (prm.s_out + BN / 2 - 1) / (BN / 2) : (prm.S + BN - 1) / BN;
+    prm.idesc |= (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    const long long total = (long long)prm.tiles_r * prm.tiles_s * prm.stacks * ksplit;
+    if (total > INT_MAX) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)total);
+    lc.blockDim = dim3(NUM_THREADS);
+    lc.dynamicSmemBytes = C::SMEM_BYTES;
+    lc.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)ksplit;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 2;
+    return cudaLaunchKernelEx(&lc, kernel, mp, mq, prm, ksplit);
+}
+
+// Clusters of `ksplit` such CTAs that the current device holds at once (0: none); asked once per device and size.
+int ksplit_capacity(int ksplit) {
+    static std::mutex mu;
+    static std::unordered_map<int, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lk(mu);
+    const int key = dev * 16 + ksplit;
+    auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    auto kernel = gemm_umma_ksplit_kernel<256, __half, false, 8>;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<256>::SMEM_BYTES) == cudaSuccess) {
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)ksplit * 148);
+        lc.blockDim = dim3(NUM_THREADS);
+        lc.dynamicSmemBytes = KsCfg<256>::SMEM_BYTES;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)ksplit;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        lc.attrs = attr;
+        lc.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+    }
+    known[key] = n;
+    return n;
+}
+
 // The output as the epilogue's TMA stores see it: [stacks][R][columns up to the end of this launch's window].
 bool make_out_maps(OutMaps *om, const UmmaParams &prm, rt_dtype dt) {
     EncodeTiledFn fn = encode_fn();
@@ -966,11 +1036,56 @@ int umma_pick_bn(long long R, long long S, long long stacks, int sm_count) {
     return 2 * t256 >= sm_count ? 256 : 128;
 }
 
+// Tile width and K split for one problem: the pair with the shortest modelled time, in SM cycles, fitted to launches of f16
+// Linears (measured back to back in one graph, us; split "128,6" = 128-column tiles, clusters of six):
+//                              1 CTA a tile    best split     neighbours
+//   [2560, 10240] x 77 rows         50.6       128,6: 15.7    128,5: 16.7  256,8: 18.1
+//   [3072, 3072]  x 40              19.4       128,4: 10.0    256,6: 10.9
+//   [384, 1536]   x 1500            12.1       128,3: 10.3    128,2: 11.8  (not split: behind fc1 in an MLP block it lost 3 %)
+//   [3072, 8192]  x 512             43.4       256,2: 37.8    128,2: 53.8
+//   [4096, 1024]  x 128, gate/up    13.9       128,4: 9.5
+//   [10240, 2560] x 128             18.4       256,3: 19.8    (80 tiles: not split)
+//   [8192, 2560]  x 200, gate/up    22.1       256,2: 24.1    (256 tiles: not split)
+// A K block costs a CTA about 520 cycles with 128 columns, 710 with 256; more when most SMs pull at once.  The split's
+// fixed part holds two cluster barriers and the exchange of its valid rows.  Clusters that do not all fit at once cost a second wave:
+// [2560, 10240] at 128,7 (140 CTAs, but 20 clusters of seven are not resident together) 26.5 us.
+void umma_pick_tile(long long R, long long S, long long K, long long stacks, bool pair, int sm_count, int *bn, int *ksplit) {
+    *bn = umma_pick_bn(R, S, stacks, sm_count);
+    *ksplit = 1;
+    const long long nk = (K + BK - 1) / BK, tiles_r = (R + BM - 1) / BM;
+    if (const char *env = getenv("RT_GEMM_KSPLIT")) { // 0: never split; "bn,split": that shape (A/B timing)
+        int fbn = 0, fsplit = 0;
+        if (sscanf(env, "%d,%d", &fbn, &fsplit) == 2 && (fbn == 128 || fbn == 256) && fsplit >= 1 && fsplit <= UMMA_KSPLIT_MAX && fsplit <= nk &&
+            (fsplit == 1 || ksplit_capacity(fsplit) > 0)) {
+            *bn = fbn;
+            *ksplit = fsplit;
+        }
+        return;
+    }
+    auto tiles_of = [&](int w) { return tiles_r * (pair ? (S / 2 + w / 2 - 1) / (w / 2) : (S + w - 1) / w) * stacks; };
+    if (4 * tiles_of(*bn) > 3 * (long long)sm_count) return; // the machine is full enough without
+    auto cost = [&](int w, int split) -> double {
+        const long long ctas = tiles_of(w) * split;
+        const long long room = split == 1 ? sm_count : (long long)split * ksplit_capacity(split);
+        if (room <= 0) return 1e30;
+        const bool busy = split > 1 && 3 * ctas > 2 * (long long)sm_count;
+        const double block = w == 128 ? (busy ? 620 : 520) : (busy ? 1100 : 710);
+        const double fixed = split == 1 ? 14000 : (w == 128 ? 13500 : 18000) + 45.0 * (double)std::min<long long>(R, BM);
+        return (double)((ctas + room - 1) / room) * (double)((nk + split - 1) / split) * block + fixed;
+    };
+    double best = cost(*bn, 1);
+    for (int w = 128; w <= 256; w *= 2)
+        for (int split = 2; split <= UMMA_KSPLIT_MAX && 4 * split <= nk; split++) {
+            const double c = cost(w, split);
+            if (c < 0.9 * best) { best = c; *bn = w; *ksplit = split; }
+        }
+}
+
 // P: [p_stack][R][K] of p_dt, Q: [q_stack][S][K] of q_dt (f16 or bf16 each); out [stacks][R][S] of out_dt.
 cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dtype q_dt, void *out, rt_dtype out_dt,
                              int R, int S, int K, int stacks, int p_stack, int q_stack, const void *bias, int bias_dt,
                              int bias_mode, int epilogue, int bn, int sm_count, cudaStream_t stream, const UmmaScatter *scatter,
-                             const float *p_scale, const float *q_scale) {
+                             const float *p_scale, const float *q_scale, int ksplit) {
     // kind::f16 wants one format for both operands: an instruction descriptor that mixes f16 and
     // bf16 is an illegal instruction on sm_100a
     if (p_dt != q_dt || (p_dt != RT_F16 && p_dt != RT_BF16)) return cudaErrorInvalidValue;
@@ -1014,6 +1129,14 @@ cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dty
     if (bn == UMMA_BN_PAIR) {
         if (out_dt == RT_F16) return launch_pair<__half>(mp, mq, prm, sm_count, stream, out_dt);
         if (out_dt == RT_BF16) return launch_pair<__nv_bfloat16>(mp, mq, prm, sm_count, stream, out_dt);
+        return cudaErrorInvalidValue;
+    }
+    if (ksplit > 1) {
+        if (out_dt == RT_F16)
+            return bn == 256 ? launch_ksplit<256, __half>(mp, mq, prm, ksplit, stream) : launch_ksplit<128, __half>(mp, mq, prm, ksplit, stream);
+        if (out_dt == RT_BF16)
+            return bn == 256 ? launch_ksplit<256, __nv_bfloat16>(mp, mq, prm, ksplit, stream)
+                             : launch_ksplit<128, __nv_bfloat16>(mp, mq, prm, ksplit, stream);
         return cudaErrorInvalidValue;
     }
     if (out_dt == RT_F16)

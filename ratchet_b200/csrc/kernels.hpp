@@ -115,10 +115,14 @@ bool umma_gemm_supported(long long K);
 // Tile width: 128 or 256 columns on one CTA per SM, or UMMA_BN_PAIR: 256 x 256 tiles on pairs of CTAs (cta_group::2)
 constexpr int UMMA_BN_PAIR = 512;
 int umma_pick_bn(long long R, long long S, long long stacks, int sm_count);
+// K split over the CTAs of a cluster (portable cluster sizes), for problems with fewer tiles than SMs
+constexpr int UMMA_KSPLIT_MAX = 8;
+void umma_pick_tile(long long R, long long S, long long K, long long stacks, bool pair, int sm_count, int *bn, int *ksplit);
 cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dtype q_dt, void *out, rt_dtype out_dt,
                              int R, int S, int K, int stacks, int p_stack, int q_stack, const void *bias, int bias_dt,
                              int bias_mode, int epilogue, int bn, int sm_count, cudaStream_t stream,
-                             const UmmaScatter *scatter = nullptr, const float *p_scale = nullptr, const float *q_scale = nullptr);
+                             const UmmaScatter *scatter = nullptr, const float *p_scale = nullptr, const float *q_scale = nullptr,
+                             int ksplit = 1);
 // (every *_bind_wait_error: the host word in which that file's kernels report a bounded wait that expired, for the current device)
 cudaError_t umma_bind_wait_error(int *word);
 

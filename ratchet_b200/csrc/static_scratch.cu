@@ -74,9 +74,10 @@ extern "C" rt_status rt_linear_q8_0_static_scratch(rt_device *dev, const void *w
     // tensor map stops at n*k: nothing left over from an earlier call is ever read, nothing needs zeroing
     e = launch_dequant(RT_Q8_0H, (long long)numel, w, scales, scratch, RT_F16, sm_count, st);
     if (e == cudaSuccess) {
-        const int bn = umma_pick_bn(rows, n, 1, sm_count);
+        int bn = 128, ksplit = 1; // the regular route's choice: the same bits
+        umma_pick_tile(rows, n, k, 1, epilogue == RT_EPILOGUE_SILU_MUL, sm_count, &bn, &ksplit);
         e = launch_gemm_umma(x, RT_F16, scratch, RT_F16, out, RT_F16, (int)rows, (int)n, (int)k, 1, 1, 1, bias, RT_F16,
-                             bias ? BIAS_PER_N : BIAS_NONE, epilogue, bn, sm_count, st);
+                             bias ? BIAS_PER_N : BIAS_NONE, epilogue, bn, sm_count, st, nullptr, nullptr, nullptr, ksplit);
     }
     if (e != cudaSuccess) return fail(RT_ERR_CUDA, std::string("rt_linear_q8_0_static_scratch launch: ") + cudaGetErrorString(e));
     return RT_OK;

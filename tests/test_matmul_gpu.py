@@ -1098,3 +1098,38 @@ def test_seeded_decode_chains_against_the_oracle(gpu, seed):
             assert np.all(np.isfinite(got)), (exe.kernel, shapes, i)
             assert oracle.rel_l2(got, oracle.f64_to_f16(truth).astype(np.float32)) <= TOL[F16], (exe.kernel, shapes, i)
             h = got
+
+
+def _check_linear(gpu, lhs_dt, act, N, K, rows, bias, epi, kernel_part):
+    """One Linear node on the expected kernel, every output against the oracle."""
+    w_t, wv = make_lhs(lhs_dt, (N, K), np.random.default_rng(5 + N), 0.05)
+    rng = np.random.default_rng(N * 7 + K * 3 + rows)
+    x = round_to(act, rng.standard_normal((1, rows, K)).astype(np.float32))
+    bdt = F16 if act == BF16 else act
+    b = round_to(bdt, rng.standard_normal(N).astype(np.float32) * 0.1) if bias else None
+    node = w_t.to(gpu).gemm(Tensor.from_data(x, gpu, act), Tensor.from_data(b, gpu, bdt) if bias else None, False, True, True, epilogue=epi)
+    name = rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()
+    assert kernel_part in name, name
+    got = node.resolve().to(Device.CPU).to_f32().reshape(rows, -1)
+    out = (lambda t: oracle.bf16_bits_to_f32(oracle.f64_to_bf16_bits(t))) if act == BF16 else (lambda t: oracle.f64_to_f16(t).astype(np.float32))
+    plain = 0 if epi == rb.EPILOGUE_SILU_MUL else epi
+    truth = oracle.matmul_truth(wv, x.reshape(rows, K), b, 1, 1, 1, N, rows, K, False, True, True, plain).reshape(rows, N)
+    if epi == rb.EPILOGUE_SILU_MUL:  # gate and up are rounded to the output's type, then folded
+        full = out(truth).astype(np.float64).reshape(rows, N)
+        gate, up = full[:, :N // 2], full[:, N // 2:]
+        truth = up * (gate / (1 + np.exp(-gate)))
+    assert oracle.rel_l2(got, out(truth).reshape(got.shape)) <= TOL[act], name
+
+
+@pytest.mark.parametrize("act,N,K,rows,bias,epi,split", [
+    (F16, 2560, 2560, 77, True, 1, "128,2"),     # ragged rows of one tile
+    (F16, 1001, 1032, 129, True, 0, "256,3"),    # ragged columns and K, a tile with one row: ranks without rows
+    (F16, 384, 1536, 1500, True, 0, "128,4"),    # several tile rows
+    (BF16, 1000, 1024, 40, False, 1, "256,8"),   # more ranks than four, bf16 output
+    (F16, 1280, 512, 200, True, 2, "128,5"),     # gate/up fold, uneven K shares
+    (BF16, 1006, 640, 33, True, 2, "256,7"),     # the fold with columns that are no multiple of 4
+])
+def test_gemm_with_k_split_over_a_cluster_matches_the_oracle(gpu, monkeypatch, act, N, K, rows, bias, epi, split):
+    monkeypatch.setenv("RT_GEMM_KSPLIT", split)
+    bn, c = split.split(",")
+    _check_linear(gpu, act, act, N, K, rows, bias, epi, f"_bn{bn}_ksplit{c}")
