@@ -69,7 +69,7 @@ struct rt_buffer {
     uint64_t klass = 0; // bytes allocated
 };
 
-enum PlanKernel { PK_GEMM_SIMT, PK_GEMV_SIMT, PK_ROWVEC_MAT, PK_Q8_GEMV_MMA, PK_Q8_GEMV_UMMA, PK_Q4K_GEMV, PK_Q4K_GEMV_UMMA, PK_GEMM_UMMA };
+enum PlanKernel { PK_GEMM_SIMT, PK_GEMV_SIMT, PK_Q8F_GEMV, PK_ROWVEC_MAT, PK_Q8_GEMV_MMA, PK_Q8_GEMV_UMMA, PK_Q4K_GEMV, PK_Q4K_GEMV_UMMA, PK_GEMM_UMMA };
 
 struct rt_plan {
     rt_device *dev = nullptr;
@@ -883,6 +883,11 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
                    (pl->bn == UMMA_BN_PAIR ? std::string("_pair256x256") : "_bn" + std::to_string(pl->bn)) +
                    (pl->ksplit > 1 ? "_ksplit" + std::to_string(pl->ksplit) : std::string()) + (pl->scratch && !pl->k_pad ? (pl->tf32x3 ? "_presplit" : "_dequant_prepass") : "") + (pl->wdq ? "_dequant_prepass" : "") +
                    (pl->rhs_transpose ? "_rhs_transposed" : "") + (pl->k_pad ? "_kpad" + std::to_string(pl->k_pad) : "");
+    } else if (s.N == 1 && !s.trans_lhs && desc->lhs_dt == RT_Q8_0F && desc->rhs_dt == RT_F32 && s.K > 0 && s.K % 32 == 0 && !empty &&
+               !force_simt()) {
+        // (whole blocks per row, so a lane's 16 codes never leave it; faster than the general GEMV at every size measured)
+        pl->kernel = PK_Q8F_GEMV;
+        pl->name = "q8f_gemv_f32";
     } else if (s.N == 1 && !s.trans_lhs) {
         pl->kernel = PK_GEMV_SIMT;
         pl->name = std::string("gemv_simt_") + dtype_name(desc->lhs_dt) + "_" + dtype_name(desc->rhs_dt);
@@ -1098,6 +1103,12 @@ static rt_status launch_node(rt_plan *plan, const void *lhs, const void *rhs, co
         if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) % 16 != 0)
             return fail(RT_ERR_ARG, "rt_matmul_launch: lhs and rhs must be 16-byte aligned");
         e = launch_q8_gemv_umma(p, plan->gemv_umma, (flags & RT_LAUNCH_LHS_CONSTANT) != 0, st);
+        break;
+    case PK_Q8F_GEMV:
+        if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) % 16 != 0) // it loads 16 bytes at a time
+            e = launch_matmul_simt(p, s.desc.lhs_dt, s.desc.rhs_dt, true, st);
+        else
+            e = launch_q8f_gemv_f32(p, (flags & RT_LAUNCH_LHS_CONSTANT) != 0, st);
         break;
     case PK_GEMV_SIMT:
         e = launch_matmul_simt(p, s.desc.lhs_dt, s.desc.rhs_dt, true, st);

@@ -1133,3 +1133,15 @@ def test_gemm_with_k_split_over_a_cluster_matches_the_oracle(gpu, monkeypatch, a
     monkeypatch.setenv("RT_GEMM_KSPLIT", split)
     bn, c = split.split(",")
     _check_linear(gpu, act, act, N, K, rows, bias, epi, f"_bn{bn}_ksplit{c}")
+
+
+@pytest.mark.parametrize("N,K,bias,epi", [(1, 32, False, 0), (5, 480, True, 1), (1003, 544, True, 0), (2560, 10240, True, 0), (4099, 5664, False, 1)])
+def test_q8f_f32_gemv_matches_the_oracle(gpu, N, K, bias, epi):
+    """Rows that are no multiple of four, a last chunk of K partly filled, one warp and ten."""
+    w_t, wv = make_lhs(Q8F, (N, K), np.random.default_rng(N + K), 0.05)
+    x = np.random.default_rng(K).standard_normal((1, 1, K)).astype(np.float32)
+    b = np.random.default_rng(N).standard_normal(N).astype(np.float32) if bias else None
+    node = w_t.to(gpu).gemm(Tensor.from_data(x, gpu, F32), Tensor.from_data(b, gpu, F32) if bias else None, False, True, True, epilogue=epi)
+    assert rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode() == "q8f_gemv_f32"
+    truth = oracle.matmul_truth(wv, x.reshape(1, K), b, 1, 1, 1, N, 1, K, False, True, True, epi)
+    assert oracle.rel_l2(node.resolve().to(Device.CPU).to_f32().reshape(-1), truth.reshape(-1).astype(np.float32)) <= TOL[F32]
