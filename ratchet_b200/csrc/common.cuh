@@ -81,10 +81,11 @@ __device__ __forceinline__ OutT epilogue_value(float acc, bool has_bias, float b
 
 // sigmoid and silu of ops/unary.rs:121-131,165-175 in f32, branch for branch: exp(v) / (1 + exp(v)) for
 // v >= 0 (which is NaN once exp(v) overflows, v > 88.7, as it is in the reference's shader), 1 / (1 + exp(-v))
-// below zero.
+// below zero.  Both are n / (1 + e) with e = exp(|v|): one exponential and one division for either sign, the same bits.
 __device__ __forceinline__ float silu_ref_f32(float v) {
-    const float sg = v >= 0.f ? expf(v) / (1.0f + expf(v)) : 1.0f / (1.0f + expf(-v));
-    return v * sg;
+    const bool pos = v >= 0.f;
+    const float e = expf(pos ? v : -v);
+    return v * ((pos ? e : 1.0f) / (1.0f + e));
 }
 
 // up * cast(silu(full(gate))) of crates/ratchet-models/src/phi3/mlp.rs:36 on values already rounded to the
