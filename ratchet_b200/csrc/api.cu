@@ -741,10 +741,12 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
         pl->kernel = PK_Q8_GEMV_MMA;
         pl->nv = (int)std::min<int64_t>(s.N, 16);
         pl->nv2 = (int)s.N - pl->nv;
-        pl->split = gemv_split;
+        const int wide = q8_gemv_mma_pick_wide(p.M, p.K, dev->sm_count, desc->lhs_dt == RT_Q8_0H ? 2 : 4, gemv_split);
+        pl->split = gemv_split | wide << 8;
         pl->launches = 1 + (pl->nv2 > 0 ? 1 : 0);
         pl->name = std::string("q8_gemv_mma_") + (desc->lhs_dt == RT_Q8_0H ? "h" : "f") + "_nv" + std::to_string(pl->nv) +
-                   (pl->nv2 ? "+" + std::to_string(pl->nv2) : std::string()) + "_split" + std::to_string(pl->split);
+                   (pl->nv2 ? "+" + std::to_string(pl->nv2) : std::string()) + "_split" + std::to_string(wide ? wide : gemv_split) +
+                   (wide ? "_rows32" : "");
     } else if (desc->lhs_dt == RT_Q4_K && desc->rhs_dt == RT_F16 && !s.trans_lhs && s.N >= 1 && s.N <= 16 &&
                (s.N == 1 || s.trans_rhs) && !empty && !force_simt() && s.stacks == 1 && q4k_umma_enabled() &&
                (double)s.M * (double)s.K >= (double)(1 << 22) &&

@@ -23,6 +23,7 @@
 //    thread-block cluster, rank 0 gathers the other CTAs' partials through distributed shared
 //    memory, also in a fixed order: results are deterministic;
 //  * epilogue = the reference's: f16(acc) + bias in f16, optional fused GELU.
+#include <algorithm>
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -69,18 +70,20 @@ __host__ __device__ inline int scale_row_stride(int nblk_slice) { return nblk_sl
 
 // Shared memory: [codes 16 x cstride][scales 16 x sstride][mbarrier]; the first 4 KB double as the
 // cross-warp reduction buffer once the codes have been consumed (the mbarrier lies beyond it).
-__host__ __device__ inline size_t bar_offset(int blocks_per_cta, int scale_size, int cols) {
-    const size_t codes = (size_t)ROWS * code_row_stride(blocks_per_cta * 32);
-    const size_t scales = ((size_t)ROWS * scale_row_stride(blocks_per_cta) * scale_size + 15) & ~(size_t)15;
-    const size_t red = (size_t)WARPS * ROWS * cols * sizeof(float);
+__host__ __device__ inline size_t bar_offset(int blocks_per_cta, int scale_size, int cols, int rows) {
+    const size_t codes = (size_t)rows * code_row_stride(blocks_per_cta * 32);
+    const size_t scales = ((size_t)rows * scale_row_stride(blocks_per_cta) * scale_size + 15) & ~(size_t)15;
+    const size_t red = (size_t)WARPS * rows * cols * sizeof(float);
     return codes + scales < red ? red : codes + scales;
 }
 
 // ScaleT: __half (Q8_0H) or float (Q8_0F).  NV: number of activation vectors, 1..8, or 16 = two groups of eight
 // MMA columns holding nv_rt (9..16) vectors.  SPLIT: K is split over a cluster of gridDim.y CTAs.
-template <typename ScaleT, int NV, bool SPLIT>
-__global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p, int blocks_per_cta, int lhs_constant, int nv_rt) {
-    constexpr int NVG = NV > 8 ? 2 : 1, COLS = NVG * 8;
+// RT: 16-row tiles per CTA.  With 9..16 vectors a block's activations (1 KB) are twice its codes (512 B per 16 rows) and do
+// not stay in what the staged weights leave of L1, so a wide weight takes two row tiles per activation load.
+template <typename ScaleT, int NV, bool SPLIT, int RT>
+__global__ void __launch_bounds__(THREADS, RT == 2 ? 3 : 5) q8_gemv_bulk_kernel(MatmulParams p, int blocks_per_cta, int lhs_constant, int nv_rt) {
+    constexpr int NVG = NV > 8 ? 2 : 1, COLS = NVG * 8, ROWS = 16 * RT;
     const int nvv = NV > 8 ? nv_rt : NV;
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p
     const int sstride = scale_row_stride(blocks_per_cta);
     uint8_t *codes_s = smem;
     ScaleT *scales_s = reinterpret_cast<ScaleT *>(smem + ROWS * cstride);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + bar_offset(blocks_per_cta, (int)sizeof(ScaleT), COLS));
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + bar_offset(blocks_per_cta, (int)sizeof(ScaleT), COLS, ROWS));
     const uint32_t bar_addr = smem_u32(bar);
 
     const int row_base = blockIdx.x * ROWS;
@@ -125,11 +128,13 @@ __global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p
     }
     {
         // 16 threads per row, no division: thread t stages scales t%16, t%16+16, ... of row t/16
-        const int r = threadIdx.x >> 4;
-        const int row = min(row_base + r, p.M - 1);
-        const ScaleT *src = scales + (long long)row * nblk + blk_begin;
-        ScaleT *dst = scales_s + r * sstride;
-        for (int j = threadIdx.x & 15; j < blk_cnt; j += 16) dst[j] = __ldg(src + j);
+#pragma unroll
+        for (int r = threadIdx.x >> 4; r < ROWS; r += THREADS / 16) {
+            const int row = min(row_base + r, p.M - 1);
+            const ScaleT *src = scales + (long long)row * nblk + blk_begin;
+            ScaleT *dst = scales_s + r * sstride;
+            for (int j = threadIdx.x & 15; j < blk_cnt; j += 16) dst[j] = __ldg(src + j);
+        }
     }
     if (lhs_constant) asm volatile("griddepcontrol.wait;" ::: "memory");
 
@@ -163,39 +168,48 @@ __global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p
         }
     }
 
-    float acc[NVG][4];
+    float acc[RT][NVG][4];
 #pragma unroll
-    for (int j = 0; j < NVG; j++)
+    for (int t = 0; t < RT; t++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc[j][i] = 0.f;
+        for (int j = 0; j < NVG; j++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[t][j][i] = 0.f;
     if (ok) {
         const uint8_t *qa = codes_s + g * cstride + c * 8;
-        const uint8_t *qb = codes_s + (g + 8) * cstride + c * 8;
-        const ScaleT *sa = scales_s + g * sstride, *sb = scales_s + (g + 8) * sstride;
+        const ScaleT *sa = scales_s + g * sstride;
 #pragma unroll 2
         for (int blk = warp; blk < blk_cnt; blk += WARPS) {
-            const uint2 wa = *reinterpret_cast<const uint2 *>(qa + blk * 32);
-            const uint2 wb = *reinterpret_cast<const uint2 *>(qb + blk * 32);
-            const float da = scale_to_f32(sa[blk]), db = scale_to_f32(sb[blk]);
-            __half2 a01, a23, a45, a67, b01, b23, b45, b67;
-            codes4_to_half2(wa.x, a01, a23);
-            codes4_to_half2(wa.y, a45, a67);
-            codes4_to_half2(wb.x, b01, b23);
-            codes4_to_half2(wb.y, b45, b67);
-            // The k index inside a block is permuted identically for W and x: lane c owns
-            // elements c*8..c*8+7; the first MMA consumes 0..3 of them, the second 4..7.
-            const uint32_t fa[4] = {h2_as_u32(a01), h2_as_u32(b01), h2_as_u32(a23), h2_as_u32(b23)};
-            const uint32_t fb[4] = {h2_as_u32(a45), h2_as_u32(b45), h2_as_u32(a67), h2_as_u32(b67)};
+            uint4 xv[NVG];
+            if (RT > 1) {
 #pragma unroll
-            for (int j = 0; j < NVG; j++) {
-                const uint4 xv = *reinterpret_cast<const uint4 *>(x[j] + blk * 32);
-                float t[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_m16n8k16_f16(t, fa, xv.x, xv.y);
-                mma_m16n8k16_f16(t, fb, xv.z, xv.w);
-                acc[j][0] = fmaf(da, t[0], acc[j][0]);
-                acc[j][1] = fmaf(da, t[1], acc[j][1]);
-                acc[j][2] = fmaf(db, t[2], acc[j][2]);
-                acc[j][3] = fmaf(db, t[3], acc[j][3]);
+                for (int j = 0; j < NVG; j++) xv[j] = *reinterpret_cast<const uint4 *>(x[j] + blk * 32);
+            }
+#pragma unroll
+            for (int t = 0; t < RT; t++) {
+                const uint2 wa = *reinterpret_cast<const uint2 *>(qa + t * 16 * cstride + blk * 32);
+                const uint2 wb = *reinterpret_cast<const uint2 *>(qa + (t * 16 + 8) * cstride + blk * 32);
+                const float da = scale_to_f32(sa[t * 16 * sstride + blk]), db = scale_to_f32(sa[(t * 16 + 8) * sstride + blk]);
+                __half2 a01, a23, a45, a67, b01, b23, b45, b67;
+                codes4_to_half2(wa.x, a01, a23);
+                codes4_to_half2(wa.y, a45, a67);
+                codes4_to_half2(wb.x, b01, b23);
+                codes4_to_half2(wb.y, b45, b67);
+                // The k index inside a block is permuted identically for W and x: lane c owns
+                // elements c*8..c*8+7; the first MMA consumes 0..3 of them, the second 4..7.
+                const uint32_t fa[4] = {h2_as_u32(a01), h2_as_u32(b01), h2_as_u32(a23), h2_as_u32(b23)};
+                const uint32_t fb[4] = {h2_as_u32(a45), h2_as_u32(b45), h2_as_u32(a67), h2_as_u32(b67)};
+#pragma unroll
+                for (int j = 0; j < NVG; j++) {
+                    if (RT == 1) xv[j] = *reinterpret_cast<const uint4 *>(x[j] + blk * 32);
+                    float s[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_m16n8k16_f16(s, fa, xv[j].x, xv[j].y);
+                    mma_m16n8k16_f16(s, fb, xv[j].z, xv[j].w);
+                    acc[t][j][0] = fmaf(da, s[0], acc[t][j][0]);
+                    acc[t][j][1] = fmaf(da, s[1], acc[t][j][1]);
+                    acc[t][j][2] = fmaf(db, s[2], acc[t][j][2]);
+                    acc[t][j][3] = fmaf(db, s[3], acc[t][j][3]);
+                }
             }
         }
     }
@@ -204,42 +218,58 @@ __global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p
     // C fragment: acc[0],acc[1] -> (row g, cols 2c,2c+1); acc[2],acc[3] -> (row g+8, same cols)
     float *red = reinterpret_cast<float *>(smem); // [WARPS][ROWS][COLS]
 #pragma unroll
-    for (int j = 0; j < NVG; j++) {
-        red[(warp * ROWS + g) * COLS + j * 8 + 2 * c] = acc[j][0];
-        red[(warp * ROWS + g) * COLS + j * 8 + 2 * c + 1] = acc[j][1];
-        red[(warp * ROWS + g + 8) * COLS + j * 8 + 2 * c] = acc[j][2];
-        red[(warp * ROWS + g + 8) * COLS + j * 8 + 2 * c + 1] = acc[j][3];
-    }
+    for (int t = 0; t < RT; t++)
+#pragma unroll
+        for (int j = 0; j < NVG; j++) {
+            float *at = red + (warp * ROWS + t * 16 + g) * COLS + j * 8 + 2 * c;
+            at[0] = acc[t][j][0];
+            at[1] = acc[t][j][1];
+            at[8 * COLS] = acc[t][j][2];
+            at[8 * COLS + 1] = acc[t][j][3];
+        }
     __syncthreads();
 
-    const int r = threadIdx.x / COLS, v = threadIdx.x % COLS; // the first ROWS * COLS threads: one (row, vector) each
-    float sum = 0.f;
-    if (threadIdx.x < ROWS * COLS) {
+    // one (row, vector) per item: the first ROWS * COLS threads, or two items per thread with two row tiles
+    constexpr int ITEMS = (ROWS * COLS + THREADS - 1) / THREADS;
+    float sum[ITEMS];
 #pragma unroll
-        for (int w = 0; w < WARPS; w++) sum += red[(w * ROWS + r) * COLS + v];
+    for (int m = 0; m < ITEMS; m++) {
+        const int item = (int)threadIdx.x + m * THREADS;
+        sum[m] = 0.f;
+        if (item < ROWS * COLS) {
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) sum[m] += red[w * ROWS * COLS + item];
+        }
     }
     if (SPLIT) {
         cg::cluster_group cluster = cg::this_cluster();
         __syncthreads();
-        if (threadIdx.x < ROWS * COLS) red[r * COLS + v] = sum;
+#pragma unroll
+        for (int m = 0; m < ITEMS; m++) {
+            const int item = (int)threadIdx.x + m * THREADS;
+            if (item < ROWS * COLS) red[item] = sum[m];
+        }
         cluster.sync();
-        if (cluster.block_rank() == 0 && threadIdx.x < ROWS * COLS) {
+        if (cluster.block_rank() == 0) {
             const unsigned n = cluster.num_blocks();
-            for (unsigned k = 1; k < n; k++) {
-                const float *remote = cluster.map_shared_rank(red, k);
-                sum += remote[r * COLS + v];
+#pragma unroll
+            for (int m = 0; m < ITEMS; m++) {
+                const int item = (int)threadIdx.x + m * THREADS;
+                if (item < ROWS * COLS)
+                    for (unsigned k = 1; k < n; k++) sum[m] += cluster.map_shared_rank(red, k)[item];
             }
         }
         cluster.sync(); // keep every CTA's shared memory alive until rank 0 has read it
         if (cluster.block_rank() != 0) return;
     }
-    if (threadIdx.x < ROWS * COLS && v < nvv) {
-        const int row = row_base + r;
-        if (row < p.M) {
+#pragma unroll
+    for (int m = 0; m < ITEMS; m++) {
+        const int item = (int)threadIdx.x + m * THREADS, r = item / COLS, v = item % COLS, row = row_base + r;
+        if (item < ROWS * COLS && v < nvv && row < p.M) {
             const bool has_bias = p.bias_mode != BIAS_NONE;
             float bias = 0.f;
             if (has_bias) bias = load_bias(p.bias, p.bias_dt, p.bias_mode == BIAS_PER_M ? row : v);
-            __half o = epilogue_value<__half>(sum, has_bias, bias, p.epilogue);
+            __half o = epilogue_value<__half>(sum[m], has_bias, bias, p.epilogue);
             // out is [stacks][M][NV] or, transposed, [stacks][NV][M]
             const long long ob = (long long)batch * p.M * nvv;
             const long long idx = p.trans_out ? ob + (long long)v * p.M + row : ob + (long long)row * nvv + v;
@@ -248,21 +278,21 @@ __global__ void __launch_bounds__(THREADS, 5) q8_gemv_bulk_kernel(MatmulParams p
     }
 }
 
-size_t smem_bytes(int blocks_per_cta, int scale_size, int cols = 8) { return bar_offset(blocks_per_cta, scale_size, cols) + 16; }
+size_t smem_bytes(int blocks_per_cta, int scale_size, int cols = 8, int rows = ROWS) { return bar_offset(blocks_per_cta, scale_size, cols, rows) + 16; }
 
-template <typename ScaleT, int NV>
+template <typename ScaleT, int NV, int RT = 1>
 cudaError_t launch_nv(const MatmulParams &p, int nv, int split, bool lhs_constant, cudaStream_t stream) {
     const int nblk = p.K / 32;
     const int bpc = (nblk + split - 1) / split;
-    const size_t smem = smem_bytes(bpc, (int)sizeof(ScaleT), NV > 8 ? 16 : 8);
-    auto kernel = split == 1 ? q8_gemv_bulk_kernel<ScaleT, NV, false> : q8_gemv_bulk_kernel<ScaleT, NV, true>;
+    const size_t smem = smem_bytes(bpc, (int)sizeof(ScaleT), NV > 8 ? 16 : 8, ROWS * RT);
+    auto kernel = split == 1 ? q8_gemv_bulk_kernel<ScaleT, NV, false, RT> : q8_gemv_bulk_kernel<ScaleT, NV, true, RT>;
     static SmemAttr smem_attr[2];
     if (smem > 48 * 1024) {
         cudaError_t e = smem_attr[split != 1].ensure(kernel, smem);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.M + ROWS - 1) / ROWS, split, p.stacks);
+    cfg.gridDim = dim3((p.M + ROWS * RT - 1) / (ROWS * RT), split, p.stacks);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -284,7 +314,8 @@ cudaError_t launch_nv(const MatmulParams &p, int nv, int split, bool lhs_constan
 }
 
 template <typename ScaleT>
-cudaError_t launch_scale(const MatmulParams &p, int nv, int split, bool lhs_constant, cudaStream_t stream) {
+cudaError_t launch_scale(const MatmulParams &p, int nv, int splits, bool lhs_constant, cudaStream_t stream) {
+    const int split = splits & 0xFF, wide = splits >> 8;
     switch (nv) {
     case 1: return launch_nv<ScaleT, 1>(p, nv, split, lhs_constant, stream);
     case 2: return launch_nv<ScaleT, 2>(p, nv, split, lhs_constant, stream);
@@ -295,7 +326,8 @@ cudaError_t launch_scale(const MatmulParams &p, int nv, int split, bool lhs_cons
     case 7: return launch_nv<ScaleT, 7>(p, nv, split, lhs_constant, stream);
     case 8: return launch_nv<ScaleT, 8>(p, nv, split, lhs_constant, stream);
     }
-    if (nv >= 9 && nv <= 16) return launch_nv<ScaleT, 16>(p, nv, split, lhs_constant, stream);
+    if (nv >= 9 && nv <= 16)
+        return wide ? launch_nv<ScaleT, 16, 2>(p, nv, wide, lhs_constant, stream) : launch_nv<ScaleT, 16>(p, nv, split, lhs_constant, stream);
     return cudaErrorInvalidValue;
 }
 
@@ -317,6 +349,29 @@ int q8_gemv_mma_pick_split(int M, int K, int sm_count, int scale_size) {
     return split;
 }
 
+// The K split for two row tiles per CTA (9..16 vectors), or 0 where one row tile is the better form.  What decides is whether
+// the CTAs are resident together (three per SM by registers, fewer by shared memory): one wave, or nearly full ones
+// where the one-tile form needs several too.  16 vectors, us, one row tile -> two: [16384, 3072] 36.9 -> 23.1 (512 CTAs on 296
+// places, split 1), [3072, 8192] 21.3 -> 13.1 (384 on 444, split 4), [3072, 1024] 7.5 -> 4.9, [1536, 3072] 8.2 -> 6.3; but
+// [10240, 2560] 13.6 -> 17.4 (320 CTAs on 296 places) and [2560, 10240] 16.3 -> 19.9, whose one-tile form is one wave.
+int q8_gemv_mma_pick_wide(int M, int K, int sm_count, int scale_size, int split) {
+    const int nblk = K / 32;
+    auto places = [&](int rows, int s, int by_regs) {
+        const size_t smem = smem_bytes((nblk + s - 1) / s, scale_size, 16, rows) + 1024; // the system's own share per CTA
+        return smem > 228 * 1024 ? 0 : sm_count * (int)std::min<size_t>(by_regs, 228 * 1024 / smem);
+    };
+    const int groups = (M + 2 * ROWS - 1) / (2 * ROWS);
+    for (int s = 1; s <= 8 && (s == 1 || nblk / s >= 2 * WARPS); s *= 2)
+        if (groups * s <= places(2 * ROWS, s, 3)) return s;
+    const int room1 = places(2 * ROWS, 1, 3), room_one_tile = places(ROWS, split, 5);
+    if (room1 > 0 && room_one_tile > 0 && (M + ROWS - 1) / ROWS * split > room_one_tile) {
+        const int waves = (groups + room1 - 1) / room1;
+        if (5 * groups >= 4 * waves * room1) return 1;
+    }
+    return 0;
+}
+
+// `splits`: the K split, and q8_gemv_mma_pick_wide's (used by 9..16 vectors) in bits 8 and up
 cudaError_t launch_q8_gemv_mma(const MatmulParams &p, bool f32_scales, int nv, int split, bool lhs_constant, cudaStream_t stream) {
     return f32_scales ? launch_scale<float>(p, nv, split, lhs_constant, stream)
                       : launch_scale<__half>(p, nv, split, lhs_constant, stream);
