@@ -113,20 +113,25 @@ __device__ __forceinline__ uint4 scaled_f16x8(const uint4 v, float down) {
 // bits (in the f16 subnormals).  scale[row] = 2^sh goes back onto the f32 accumulators in the GEMM's epilogue: both
 // multiplications are exact.  Infinities and NaNs pass through as they are; a row without a finite non-zero element
 // has the factor 1.
+// TEAM: warps per row (1, or 4 for rows past 4096 values).
+template <int TEAM>
 __global__ void __launch_bounds__(256) cast_bf16_f16_rows_kernel(const __nv_bfloat16 *__restrict__ src, __half *__restrict__ dst,
                                                                  float *__restrict__ scale, long long rows, int K) {
     // the next kernel may start its prologue now; this one's stream predecessor may still be reading what it writes
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // One warp per row: the row's largest magnitude needs shuffles only, and rows of up to 4096 values (16 loads of
-    // 16 bytes per lane, all in flight together) stay in registers between the two steps; longer rows are read a
-    // second time, out of L2.
-    constexpr int HOLD = 16;
-    const int lane = threadIdx.x & 31;
-    const long long warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5), n_warps = (long long)gridDim.x * 8;
+    // Rows of up to 4096 values take one warp, longer ones four that meet in shared memory for the row's largest
+    // magnitude; up to 16 loads of 16 bytes per lane, all in flight together, stay in registers between the two steps.  Only
+    // rows past 16384 values are read a second time (one warp per row read 10240 values twice: 84 us for 8192 rows, whose
+    // one reading and one writing take 50).
+    constexpr int HOLD = 16, LANES = TEAM * 32;
+    __shared__ float team_max[2][8];
+    const int lane = threadIdx.x % LANES, in_block = threadIdx.x / LANES;
+    const long long warp = (long long)blockIdx.x * (8 / TEAM) + in_block, n_warps = (long long)gridDim.x * (8 / TEAM);
+    int turn = 0;
     const bool vec = (K % 8) == 0; // then every row starts on a 16-byte boundary
     const int n8 = vec ? K / 8 : 0;
-    const bool held = n8 <= HOLD * 32;
+    const bool held = n8 <= HOLD * LANES;
     for (long long r = warp; r < rows; r += n_warps) {
         const __nv_bfloat16 *s = src + r * K;
         __half *d = dst + r * K;
@@ -135,20 +140,27 @@ __global__ void __launch_bounds__(256) cast_bf16_f16_rows_kernel(const __nv_bflo
         if (held) {
 #pragma unroll
             for (int j = 0; j < HOLD; j++) {
-                const int i = lane + 32 * j;
+                const int i = lane + LANES * j;
                 keep[j] = i < n8 ? __ldg(reinterpret_cast<const uint4 *>(s) + i) : make_uint4(0, 0, 0, 0);
             }
 #pragma unroll
             for (int j = 0; j < HOLD; j++) m = fmaxf(m, finite_amax8(keep[j]));
         } else {
-            for (int i = lane; i < n8; i += 32) m = fmaxf(m, finite_amax8(__ldg(reinterpret_cast<const uint4 *>(s) + i)));
+            for (int i = lane; i < n8; i += LANES) m = fmaxf(m, finite_amax8(__ldg(reinterpret_cast<const uint4 *>(s) + i)));
         }
-        for (int i = n8 * 8 + lane; i < K; i += 32) {
+        for (int i = n8 * 8 + lane; i < K; i += LANES) {
             const float a = fabsf(__bfloat162float(s[i]));
             if (a <= 3.0e38f) m = fmaxf(m, a);
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (TEAM > 1) { // the two buffers alternate: a warp writes one again only after the barrier of the row between
+            if ((threadIdx.x & 31) == 0) team_max[turn][threadIdx.x >> 5] = m;
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + in_block), "n"(LANES) : "memory");
+#pragma unroll
+            for (int w = 0; w < TEAM; w++) m = fmaxf(m, team_max[turn][in_block * TEAM + w]);
+            turn ^= 1;
+        }
         int sh = 0;
         if (m > 0.f) {
             int e;
@@ -159,14 +171,14 @@ __global__ void __launch_bounds__(256) cast_bf16_f16_rows_kernel(const __nv_bflo
         if (held) {
 #pragma unroll
             for (int j = 0; j < HOLD; j++) {
-                const int i = lane + 32 * j;
+                const int i = lane + LANES * j;
                 if (i < n8) reinterpret_cast<uint4 *>(d)[i] = scaled_f16x8(keep[j], down);
             }
         } else {
-            for (int i = lane; i < n8; i += 32)
+            for (int i = lane; i < n8; i += LANES)
                 reinterpret_cast<uint4 *>(d)[i] = scaled_f16x8(__ldg(reinterpret_cast<const uint4 *>(s) + i), down);
         }
-        for (int i = n8 * 8 + lane; i < K; i += 32) d[i] = __float2half_rn(__bfloat162float(s[i]) * down);
+        for (int i = n8 * 8 + lane; i < K; i += LANES) d[i] = __float2half_rn(__bfloat162float(s[i]) * down);
         if (lane == 0) scale[r] = ldexpf(1.f, sh);
     }
 }
@@ -267,9 +279,10 @@ cudaError_t launch_silu_mul(const void *full, void *out, long long rows, int ff,
 
 cudaError_t launch_cast_bf16_f16_rows(const void *src, void *dst, float *scale, long long rows, int K, int sm_count, cudaStream_t stream) {
     if (rows == 0 || K == 0) return cudaSuccess;
-    const long long want = (rows + 7) / 8; // eight rows (warps) per block
+    const int team = K > 4096 ? 4 : 1, per_block = 8 / team; // rows at a time
+    const long long want = (rows + per_block - 1) / per_block;
     const int blocks = (int)(want < (long long)sm_count * 8 ? want : (long long)sm_count * 8);
-    return launch_pdl(cast_bf16_f16_rows_kernel, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16 *)src, (__half *)dst, scale, rows, K);
+    return launch_pdl(team == 4 ? cast_bf16_f16_rows_kernel<4> : cast_bf16_f16_rows_kernel<1>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16 *)src, (__half *)dst, scale, rows, K);
 }
 
 cudaError_t launch_dequant(rt_dtype dt, long long numel, const void *src, const void *scales, void *dst, rt_dtype out_dt,
