@@ -372,6 +372,76 @@ __device__ __forceinline__ void epilogue_tile(const UmmaParams &prm, uint32_t tm
     }
 }
 
+// The epilogue of a tile with the gate/up fold (accumulator columns 0 .. BN/2-1 gate, BN/2 .. BN-1 up), for both kernels.
+template <int BN, typename OutT, bool REMOTE_DONE>
+__device__ __forceinline__ void epilogue_fold_tile(const UmmaParams &prm, uint32_t tmem_acc, uint32_t bar_done, int r0, int s0, int b, int q, int half,
+                                                   int lane, uint8_t *stg, const float *bias_s, bool has_bias, float row_mul, bool vec_ok) {
+    // 32 output columns per round: the gate accumulators, the up accumulators BN/2 columns further on,
+    // up * silu(gate), then out through the staging rows (four 16-byte chunks each)
+#pragma unroll 1
+    for (int cc = half; cc < BN / 64; cc += 2) {
+        const int colbase = s0 + cc * 32;
+        uint32_t vg[32], vu[32];
+        tmem_ld32(tmem_acc + cc * 32 + ((uint32_t)(q * 32) << 16), vg);
+        tmem_ld32(tmem_acc + BN / 2 + cc * 32 + ((uint32_t)(q * 32) << 16), vu);
+        if (cc + 2 >= BN / 64) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                if (REMOTE_DONE) arrive_cluster(bar_done);
+                else mbar_arrive(bar_done);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                float o[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int i = g * 8 + j * 2 + e;
+                    const float bg = has_bias ? bias_s[cc * 32 + i] : 0.f;
+                    const float bu = has_bias ? bias_s[BN / 2 + cc * 32 + i] : 0.f;
+                    const float ga = HAS_OPERAND_FACTORS<OutT> ? __uint_as_float(vg[i]) * row_mul : __uint_as_float(vg[i]);
+                    const float ua = HAS_OPERAND_FACTORS<OutT> ? __uint_as_float(vu[i]) * row_mul : __uint_as_float(vu[i]);
+                    const OutT gv = epilogue_value<OutT>(ga, has_bias, bg, RT_EPILOGUE_NONE);
+                    const OutT uv = epilogue_value<OutT>(ua, has_bias, bu, RT_EPILOGUE_NONE);
+                    o[e] = to_f32(silu_mul_value<OutT>(gv, uv));
+                }
+                w[j] = pack2<OutT>(o[0], o[1]);
+            }
+            *reinterpret_cast<uint4 *>(stg + lane * STG_ROW_BYTES + ((g ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        __syncwarp();
+        if (vec_ok) {
+            const int colv = colbase + (lane & 3) * 8;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int rl = 8 * i + (lane >> 2);
+                const int rg = r0 + q * 32 + rl;
+                if (rg < prm.R && colv < prm.s_out) {
+                    const uint4 pk = *reinterpret_cast<const uint4 *>(stg + rl * STG_ROW_BYTES + (((lane & 3) ^ (rl & 7)) << 4));
+                    const long long off = (long long)b * prm.out_batch_stride + (long long)rg * prm.out_ld + prm.out_col + colv;
+                    for (int d = 0; d < prm.n_out; d++) *reinterpret_cast<uint4 *>(reinterpret_cast<OutT *>(prm.outs[d]) + off) = pk;
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (int rl = 0; rl < 32; rl++) {
+                const int rg = r0 + q * 32 + rl;
+                if (rg >= prm.R) break;
+                if (colbase + lane < prm.s_out) {
+                    const OutT o = *reinterpret_cast<const OutT *>(stg + rl * STG_ROW_BYTES + (((lane >> 3) ^ (rl & 7)) << 4) + (lane & 7) * 2);
+                    const long long off = (long long)b * prm.out_batch_stride + (long long)rg * prm.out_ld + prm.out_col + colbase + lane;
+                    for (int d = 0; d < prm.n_out; d++) reinterpret_cast<OutT *>(prm.outs[d])[off] = o;
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // PAIR: the gate/up fold of RT_EPILOGUE_SILU_MUL (see UmmaParams::pair), compiled only into the kernels that run it
 template <int BN, typename OutT, bool PAIR>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -515,67 +585,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
             // 128-byte line per row (this matters most when the destination is a peer GPU over NVLink)
             uint8_t *stg = stage_out + (warp - 2) * (32 * STG_ROW_BYTES);
             if (PAIR) {
-                // 32 output columns per round: the gate accumulators, the up accumulators BN/2 columns further on,
-                // up * silu(gate), then out through the staging rows (four 16-byte chunks each)
-#pragma unroll 1
-                for (int cc = half; cc < BN / 64; cc += 2) {
-                    const int colbase = s0 + cc * 32;
-                    uint32_t vg[32], vu[32];
-                    tmem_ld32(tmem_base + acc * BN + cc * 32 + ((uint32_t)(q * 32) << 16), vg);
-                    tmem_ld32(tmem_base + acc * BN + BN / 2 + cc * 32 + ((uint32_t)(q * 32) << 16), vu);
-                    if (cc + 2 >= BN / 64) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
-                    }
-#pragma unroll
-                    for (int g = 0; g < 4; g++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            float o[2];
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                const int i = g * 8 + j * 2 + e;
-                                const float bg = has_bias ? bias_s[cc * 32 + i] : 0.f;
-                                const float bu = has_bias ? bias_s[BN / 2 + cc * 32 + i] : 0.f;
-                                const float ga = HAS_OPERAND_FACTORS<OutT> ? __uint_as_float(vg[i]) * row_mul : __uint_as_float(vg[i]);
-                                const float ua = HAS_OPERAND_FACTORS<OutT> ? __uint_as_float(vu[i]) * row_mul : __uint_as_float(vu[i]);
-                                const OutT gv = epilogue_value<OutT>(ga, has_bias, bg, RT_EPILOGUE_NONE);
-                                const OutT uv = epilogue_value<OutT>(ua, has_bias, bu, RT_EPILOGUE_NONE);
-                                o[e] = to_f32(silu_mul_value<OutT>(gv, uv));
-                            }
-                            w[j] = pack2<OutT>(o[0], o[1]);
-                        }
-                        *reinterpret_cast<uint4 *>(stg + lane * STG_ROW_BYTES + ((g ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                    __syncwarp();
-                    if (vec_ok) {
-                        const int colv = colbase + (lane & 3) * 8;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const int rl = 8 * i + (lane >> 2);
-                            const int rg = r0 + q * 32 + rl;
-                            if (rg < prm.R && colv < prm.s_out) {
-                                const uint4 pk = *reinterpret_cast<const uint4 *>(stg + rl * STG_ROW_BYTES + (((lane & 3) ^ (rl & 7)) << 4));
-                                const long long off = (long long)b * prm.out_batch_stride + (long long)rg * prm.out_ld + prm.out_col + colv;
-                                for (int d = 0; d < prm.n_out; d++) *reinterpret_cast<uint4 *>(reinterpret_cast<OutT *>(prm.outs[d]) + off) = pk;
-                            }
-                        }
-                    } else {
-#pragma unroll 4
-                        for (int rl = 0; rl < 32; rl++) {
-                            const int rg = r0 + q * 32 + rl;
-                            if (rg >= prm.R) break;
-                            if (colbase + lane < prm.s_out) {
-                                const OutT o = *reinterpret_cast<const OutT *>(stg + rl * STG_ROW_BYTES + (((lane >> 3) ^ (rl & 7)) << 4) + (lane & 7) * 2);
-                                const long long off = (long long)b * prm.out_batch_stride + (long long)rg * prm.out_ld + prm.out_col + colbase + lane;
-                                for (int d = 0; d < prm.n_out; d++) reinterpret_cast<OutT *>(prm.outs[d])[off] = o;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
+                epilogue_fold_tile<BN, OutT, false>(prm, tmem_base + acc * BN, bar_tempty + 8 * acc, r0, s0, b, q, half, lane, stg, bias_s, has_bias,
+                                                    row_mul, vec_ok);
                 if (++acc == 2) { acc = 0; acc_phase ^= 1; }
                 continue;
             }
@@ -648,7 +659,9 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                  : "memory");
 }
 
-template <typename OutT>
+// FOLD (the gate/up fold): a tile is 128 output columns; the leading CTA loads their 128 gate rows of Q, the other one the
+// 128 up rows, which the MMA reads as columns 0 .. 127 and 128 .. 255 of one 256-column tile.
+template <typename OutT, bool FOLD>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ OutMaps omaps,
                       const UmmaParams prm) {
@@ -707,7 +720,8 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_co
                 const int b = tile / tiles_per_batch, rem = tile % tiles_per_batch;
                 int tr, ts;
                 tile_coords(rem, prm.tiles_r, prm.tiles_s, prm.group_r, tr, ts);
-                const int r0 = tr * 2 * BM + (int)rank * BM, s0 = ts * BN + (int)rank * (BN / 2);
+                const int r0 = tr * 2 * BM + (int)rank * BM;
+                const int s0 = FOLD ? ts * (BN / 2) + (int)rank * prm.s_out : ts * BN + (int)rank * (BN / 2);
                 const int bp = b % prm.p_stack, bq = b % prm.q_stack;
                 for (int kb = 0; kb < num_k; kb++) {
                     if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, 1)) { ok = false; break; }
@@ -767,11 +781,14 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_co
             const int b = tile / tiles_per_batch, rem = tile % tiles_per_batch;
             int tr, ts;
             tile_coords(rem, prm.tiles_r, prm.tiles_s, prm.group_r, tr, ts);
-            const int r0 = tr * 2 * BM + (int)rank * BM, s0 = ts * BN;
+            const int r0 = tr * 2 * BM + (int)rank * BM, s0 = ts * (FOLD ? BN / 2 : BN);
             if (bar_red_or(1, EPI_WARPS * 32, gave_up || *abort_flag != 0)) break;
             if (prm.bias_mode == BIAS_PER_N) {
-                for (int j = ep_tid; j < BN; j += EPI_WARPS * 32)
-                    bias_s[j] = (s0 + j < prm.S) ? load_bias(prm.bias, prm.bias_dt, s0 + j) : 0.f;
+                for (int j = ep_tid; j < BN; j += EPI_WARPS * 32) {
+                    const int jj = FOLD ? j % (BN / 2) : j;
+                    const int wrow = FOLD ? (j / (BN / 2)) * prm.s_out + s0 + jj : s0 + j;
+                    bias_s[j] = (s0 + jj < prm.s_out) ? load_bias(prm.bias, prm.bias_dt, wrow) : 0.f;
+                }
             }
             asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
             if (!mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, 4)) { gave_up = true; continue; }
@@ -782,7 +799,10 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_co
             if (prm.bias_mode == BIAS_PER_M && row < prm.R) row_bias = load_bias(prm.bias, prm.bias_dt, row);
             const float row_mul = (HAS_OPERAND_FACTORS<OutT> && prm.p_scale && row < prm.R) ? __ldg(prm.p_scale + (long long)(b % prm.p_stack) * prm.R + row) : 1.f;
             uint8_t *stg = stage_out + (warp - 2) * (32 * STG_ROW_BYTES);
-            epilogue_tile<BN, OutT, true, true>(prm, tmem_base + acc * BN, tempty0 + 8 * acc, r0, s0, b, q, half, lane, stg, bias_s, has_bias, row_bias,
+            if (FOLD)
+                epilogue_fold_tile<BN, OutT, true>(prm, tmem_base + acc * BN, tempty0 + 8 * acc, r0, s0, b, q, half, lane, stg, bias_s, has_bias, row_mul,
+                                                   vec_ok);
+            else epilogue_tile<BN, OutT, true, true>(prm, tmem_base + acc * BN, tempty0 + 8 * acc, r0, s0, b, q, half, lane, stg, bias_s, has_bias, row_bias,
                                                 row_mul, vec_ok, pair_ok, &omaps);
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
@@ -990,15 +1010,15 @@ bool make_out_maps(OutMaps *om, const UmmaParams &prm, rt_dtype dt) {
 
 template <typename OutT>
 cudaError_t launch_pair(const CUtensorMap &mp, const CUtensorMap &mq, UmmaParams prm, int sm_count, cudaStream_t stream, rt_dtype out_dt) {
-    static SmemAttr smem_attr;
-    auto kernel = gemm_umma_pair_kernel<OutT>;
+    static SmemAttr smem_attr[2];
+    auto kernel = prm.pair ? gemm_umma_pair_kernel<OutT, true> : gemm_umma_pair_kernel<OutT, false>;
     {
-        cudaError_t e = smem_attr.ensure(kernel, P2_SMEM_BYTES);
+        cudaError_t e = smem_attr[prm.pair].ensure(kernel, P2_SMEM_BYTES);
         if (e != cudaSuccess) return e;
     }
     prm.tiles_r = (prm.R + 2 * BM - 1) / (2 * BM);
     prm.group_r = grouped_order(prm) ? TILE_GROUP_ROWS / (2 * BM) : prm.tiles_r;
-    prm.tiles_s = (prm.S + P2_BN - 1) / P2_BN;
+    prm.tiles_s = prm.pair ? (prm.s_out + P2_BN / 2 - 1) / (P2_BN / 2) : (prm.S + P2_BN - 1) / P2_BN;
     // instruction descriptor: f32 accumulate, K-major A and B, N = 256, M = 256 over the two CTAs
     prm.idesc |= (1u << 4) | ((uint32_t)(P2_BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
     const long long total = (long long)prm.tiles_r * prm.tiles_s * prm.stacks;
@@ -1021,7 +1041,7 @@ cudaError_t launch_pair(const CUtensorMap &mp, const CUtensorMap &mq, UmmaParams
     static const bool tma_store_wanted = [] { const char *v = getenv("RT_GEMM_TMA_STORE"); return !(v && v[0] == '0'); }();
     OutMaps om;
     memset(&om, 0, sizeof(om));
-    prm.tma_store = tma_store_wanted && make_out_maps(&om, prm, out_dt) ? 1 : 0;
+    prm.tma_store = tma_store_wanted && !prm.pair && make_out_maps(&om, prm, out_dt) ? 1 : 0;
     return cudaLaunchKernelEx(&lc, kernel, mp, mq, om, prm);
 }
 
@@ -1093,8 +1113,7 @@ cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dty
     if (pair && (S % 2 != 0 || bias_mode == BIAS_PER_M || (scatter && scatter->n_out > 0))) return cudaErrorInvalidValue;
     CUtensorMap mp, mq;
     if (!make_map(&mp, P, p_dt, K, R, p_stack, BM)) return cudaErrorInvalidValue;
-    if (bn == UMMA_BN_PAIR && pair) return cudaErrorInvalidValue; // the CTA-pair kernel has no gate/up fold
-    if (!(pair ? make_pair_map(&mq, Q, q_dt, K, S / 2, q_stack, bn / 2)
+    if (!(pair && bn != UMMA_BN_PAIR ? make_pair_map(&mq, Q, q_dt, K, S / 2, q_stack, bn / 2)
                : make_map(&mq, Q, q_dt, K, S, q_stack, bn == UMMA_BN_PAIR ? P2_BN / 2 : bn)))
         return cudaErrorInvalidValue;
     UmmaParams prm{};

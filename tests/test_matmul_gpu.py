@@ -1145,3 +1145,21 @@ def test_q8f_f32_gemv_matches_the_oracle(gpu, N, K, bias, epi):
     assert rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode() == "q8f_gemv_f32"
     truth = oracle.matmul_truth(wv, x.reshape(1, K), b, 1, 1, 1, N, 1, K, False, True, True, epi)
     assert oracle.rel_l2(node.resolve().to(Device.CPU).to_f32().reshape(-1), truth.reshape(-1).astype(np.float32)) <= TOL[F32]
+
+
+@pytest.mark.parametrize("act,wshape,rows,bias", [
+    (F16, (2 * 4096, 2048), 300, True),       # the second tile row ends in a pair's first CTA
+    (BF16, (2 * 4000, 2080), 513, False),     # a last tile of 32 of its 128 columns: gate rows past the half are up rows
+])
+def test_gate_up_fold_on_cta_pairs_has_the_bits_of_the_single_cta_kernel(gpu, monkeypatch, act, wshape, rows, bias):
+    rng = np.random.default_rng(rows)
+    w = Tensor.from_data(round_to(act, rng.standard_normal(wshape).astype(np.float32) * 0.02), gpu, act)
+    x = Tensor.from_data(round_to(act, rng.standard_normal((1, rows, wshape[1])).astype(np.float32)), gpu, act)
+    b = Tensor.from_data(round_to(F16, rng.standard_normal(wshape[0]).astype(np.float32) * 0.1), gpu, F16) if bias else None
+    got = []
+    for pair in ("1", "0"):
+        monkeypatch.setenv("RT_GEMM_PAIR", pair)
+        node = w.gemm(x, b, False, True, True, epilogue=rb.EPILOGUE_SILU_MUL)
+        assert ("pair256x256" in rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()) == (pair == "1")
+        got.append(node.resolve().to(Device.CPU).to_numpy())
+    assert np.array_equal(got[0], got[1])
