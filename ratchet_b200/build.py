@@ -27,7 +27,7 @@ SOURCES = [
     "gemv_q8_mma.cu",
     "gemv_q8_umma.cu", "gemv_q8_chain.cu",
     "gemv_q4k_mma.cu", "gemv_q4k_umma.cu",
-    "gemv_q8f_f32.cu",
+    "gemv_q8f_f32.cu", "gemv_q4k_f16.cu",
     "dequant.cu",
     "gemm_umma.cu", "gemm_umma_tf32.cu",
     "static_scratch.cu",

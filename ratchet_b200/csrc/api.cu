@@ -69,7 +69,7 @@ struct rt_buffer {
     uint64_t klass = 0; // bytes allocated
 };
 
-enum PlanKernel { PK_GEMM_SIMT, PK_GEMV_SIMT, PK_Q8F_GEMV, PK_ROWVEC_MAT, PK_Q8_GEMV_MMA, PK_Q8_GEMV_UMMA, PK_Q4K_GEMV, PK_Q4K_GEMV_UMMA, PK_GEMM_UMMA };
+enum PlanKernel { PK_GEMM_SIMT, PK_GEMV_SIMT, PK_Q8F_GEMV, PK_Q4K_GEMV_F16, PK_ROWVEC_MAT, PK_Q8_GEMV_MMA, PK_Q8_GEMV_UMMA, PK_Q4K_GEMV, PK_Q4K_GEMV_UMMA, PK_GEMM_UMMA };
 
 struct rt_plan {
     rt_device *dev = nullptr;
@@ -747,6 +747,13 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
         pl->name = std::string("q8_gemv_mma_") + (desc->lhs_dt == RT_Q8_0H ? "h" : "f") + "_nv" + std::to_string(pl->nv) +
                    (pl->nv2 ? "+" + std::to_string(pl->nv2) : std::string()) + "_split" + std::to_string(wide ? wide : gemv_split) +
                    (wide ? "_rows32" : "");
+    } else if (desc->lhs_dt == RT_Q4_K && desc->rhs_dt == RT_F16 && !s.trans_lhs && s.N == 1 && s.K > 0 && s.K % 256 == 0 && !empty && !force_simt() &&
+               getenv("RT_Q4K_UMMA") == nullptr && !(s.K > 2048 && (q4k_gemv_pick_split(p.M, p.K, 1, (int)s.stacks, dev->sm_count) & 0xff) == 1)) {
+        // one vector: registers only (RT_Q4K_UMMA=1 / 0 picks the tensor-memory or the warp-MMA kernel instead).  The warp-MMA
+        // kernel keeps the long rows of which one CTA holds all K and which fill the machine without a K split:
+        // [10240, 2560] 11.0 against 11.8 us, [16384, 3072] with the fold 16.8 against 17.8.
+        pl->kernel = PK_Q4K_GEMV_F16;
+        pl->name = "q4k_gemv_f16";
     } else if (desc->lhs_dt == RT_Q4_K && desc->rhs_dt == RT_F16 && !s.trans_lhs && s.N >= 1 && s.N <= 16 &&
                (s.N == 1 || s.trans_rhs) && !empty && !force_simt() && s.stacks == 1 && q4k_umma_enabled() &&
                (double)s.M * (double)s.K >= (double)(1 << 22) &&
@@ -901,7 +908,9 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
         pl->name = std::string("gemm_simt_") + dtype_name(desc->lhs_dt) + "_" + dtype_name(desc->rhs_dt);
     }
     if (s.epilogue == RT_EPILOGUE_SILU_MUL) {
-        if (pl->kernel == PK_GEMM_UMMA && !pl->tf32x3) {
+        if (pl->kernel == PK_Q4K_GEMV_F16) {
+            pl->name += "+silu_mul"; // a CTA holds gate rows and their up rows
+        } else if (pl->kernel == PK_GEMM_UMMA && !pl->tf32x3) {
             pl->name += "_silu_mul_paired_tiles"; // gate and up rows of a column meet in one tile
         } else {
             pl->pair = true;
@@ -1093,6 +1102,11 @@ static rt_status launch_node(rt_plan *plan, const void *lhs, const void *rhs, co
             const int nv = std::min(16, plan->nv + plan->nv2 - done);
             e = launch_q8_gemv_mma(p2, s.desc.lhs_dt == RT_Q8_0F, nv, plan->split, (flags & RT_LAUNCH_LHS_CONSTANT) != 0, st);
         }
+        break;
+    case PK_Q4K_GEMV_F16:
+        if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) % 16 != 0)
+            return fail(RT_ERR_ARG, "rt_matmul_launch: lhs and rhs must be 16-byte aligned");
+        e = launch_q4k_gemv_f16(p, s.epilogue == RT_EPILOGUE_SILU_MUL, (flags & RT_LAUNCH_LHS_CONSTANT) != 0, st);
         break;
     case PK_Q4K_GEMV:
         if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) % 16 != 0)

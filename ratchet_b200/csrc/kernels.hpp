@@ -50,6 +50,8 @@ class SmemAttr {
 cudaError_t launch_matmul_simt(const MatmulParams &p, rt_dtype lhs_dt, rt_dtype act_dt, bool gemv, cudaStream_t stream);
 // Q8_0F x f32, one vector, K % 32 == 0, operands 16-byte aligned
 cudaError_t launch_q8f_gemv_f32(const MatmulParams &p, bool lhs_constant, cudaStream_t stream);
+// Q4_K x f16, one vector, operands 16-byte aligned; silu_pairs: lhs rows are gate | up, the output their fold
+cudaError_t launch_q4k_gemv_f16(const MatmulParams &p, bool silu_pairs, bool lhs_constant, cudaStream_t stream);
 // one row of a dense lhs against a dense rhs stored [K][N] of the same dtype (M == 1, no transposes)
 int rowvec_mat_chunks(int N, int K, int stacks, int sm_count); // CTAs that share the k rows (1: no partial sums)
 cudaError_t launch_rowvec_mat(const MatmulParams &p, rt_dtype dt, int chunks, float *partial, cudaStream_t stream);

@@ -1163,3 +1163,22 @@ def test_gate_up_fold_on_cta_pairs_has_the_bits_of_the_single_cta_kernel(gpu, mo
         assert ("pair256x256" in rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()) == (pair == "1")
         got.append(node.resolve().to(Device.CPU).to_numpy())
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("N,K,bias,epi", [(1, 256, False, 0), (5, 1024, True, 1), (1003, 3072, True, 0), (2562, 8448, True, 0), (2 * 501, 1280, True, 2),
+                                          (2, 512, False, 2)])
+def test_q4k_f16_gemv_matches_the_oracle(gpu, N, K, bias, epi):
+    """Rows that are no multiple of four, gate rows that are no multiple of two, one warp and more steps than warps."""
+    _check_linear(gpu, Q4K, F16, N, K, 1, bias, epi, "q4k_gemv_f16")
+
+
+def test_q4k_f16_gemv_with_infinities_and_nan(gpu):
+    """An infinity against weights of one sign and a NaN come out as the plain f32 sum gives them."""
+    w_t, wv = make_lhs(Q4K, (64, 512), np.random.default_rng(3), 0.05)
+    for value in (np.inf, -np.inf, np.nan):
+        x = round_to(F16, np.random.default_rng(4).standard_normal((1, 1, 512)).astype(np.float32))
+        x[0, 0, 77] = value
+        got = w_t.to(gpu).gemm(Tensor.from_data(x, gpu, F16), None, False, True, True).resolve().to(Device.CPU).to_f32().reshape(-1)
+        with np.errstate(invalid="ignore"):
+            want = wv.reshape(64, 512)[:, 77] * np.float32(value)
+        assert np.array_equal(got, want, equal_nan=True)
