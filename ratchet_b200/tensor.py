@@ -100,6 +100,7 @@ class Device:
         self.ordinal = ordinal
         self._h = handle
         self._plans = {}
+        self._form_plans = {}  # (node form, routing stamp) -> plan
 
     @classmethod
     def request_device(cls, req: DeviceRequest, ordinal: Optional[int] = None) -> "Device":
@@ -200,11 +201,12 @@ class GpuBuffer:
 
 
 class _NodeForm:
-    """What a Matmul node is apart from its data: its description, what the library's rules say of it, and its plans.
+    """What a Matmul node is apart from its data: its description and what the library's rules say of it.
     Pure functions of dtypes, shapes and flags, so equal nodes share one (a decode step asks for the same few forms token
-    after token; working one out again costs more than launching its kernel)."""
+    after token; working one out again costs more than launching its kernel).  A form's plans stay with the Device they
+    were made on: they end with it."""
 
-    __slots__ = ("desc", "spec", "out_shape", "out_dt", "_plans")
+    __slots__ = ("desc", "spec", "out_shape", "out_dt")
     _known: dict = {}
     LIMIT = 4096  # forms kept; a program with more distinct shapes starts over
 
@@ -215,7 +217,6 @@ class _NodeForm:
         check(_lib.load().rt_matmul_spec(byref(desc), byref(self.spec)))
         self.out_shape = self.spec.out_shape.tolist()
         self.out_dt = _DTYPES[self.spec.out_dt]
-        self._plans = {}
 
     @classmethod
     def of(cls, op: "Matmul") -> "_NodeForm":
@@ -231,10 +232,12 @@ class _NodeForm:
         return form
 
     def plan(self, device: Device, stamp: int) -> int:
-        key = (device._h.value, stamp)
-        h = self._plans.get(key)
+        plans = device._form_plans
+        h = plans.get((self, stamp))
         if h is None:
-            h = self._plans[key] = device.plan_for(self.desc).value
+            if len(plans) >= self.LIMIT:
+                plans.clear()
+            h = plans[self, stamp] = device.plan_for(self.desc).value
         return h
 
 

@@ -323,3 +323,25 @@ def test_oracle_silu_follows_the_two_branch_sigmoid():
     got = oracle.silu_mul(full, "f16")
     want = np.array([[3.0 * np.float16(0.7310586), 0.5 * np.float16(-2.0 * 0.11920292)]], dtype=np.float16)
     assert np.array_equal(got.astype(np.float16), want)
+
+
+def test_plans_of_a_node_form_stay_with_the_device_they_were_made_on(monkeypatch):
+    """A device destroyed and another created at the same address: the second one plans for itself (the first one's plans
+    were freed with it)."""
+    made = []
+    monkeypatch.setattr(rb.Device, "plan_for", lambda self, desc: made.append(self) or ctypes.c_void_p(0x1000 * len(made)))
+    x, w = Tensor.from_data(np.zeros((1, 3, 8), np.float32)), Tensor.from_data(np.zeros((5, 8), np.float32))
+    form = w.gemm(x, None, False, True, True).op._form
+    first, second = (rb.Device(rb.DeviceRequest.GPU, 0, ctypes.c_void_p(0x7000)) for _ in range(2))
+    assert form.plan(first, 1) == form.plan(first, 1) == 0x1000
+    assert form.plan(second, 1) == 0x2000 and form.plan(second, 2) == 0x3000
+    assert made == [first, second, second]
+
+
+def test_plans_kept_per_device_are_bounded(monkeypatch):
+    monkeypatch.setattr(rb.Device, "plan_for", lambda self, desc: ctypes.c_void_p(0x1000))
+    form = Tensor.from_data(np.zeros((5, 8), np.float32)).gemm(Tensor.from_data(np.zeros((1, 3, 8), np.float32)), None, False, True, True).op._form
+    device = rb.Device(rb.DeviceRequest.GPU, 0, ctypes.c_void_p(0x7000))
+    for stamp in range(2 * form.LIMIT + 3):
+        form.plan(device, stamp)
+    assert len(device._form_plans) <= form.LIMIT
