@@ -741,7 +741,7 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
         pl->kernel = PK_Q8_GEMV_MMA;
         pl->nv = (int)std::min<int64_t>(s.N, 16);
         pl->nv2 = (int)s.N - pl->nv;
-        const int wide = q8_gemv_mma_pick_wide(p.M, p.K, dev->sm_count, desc->lhs_dt == RT_Q8_0H ? 2 : 4, gemv_split);
+        const int wide = q8_gemv_mma_pick_wide(p.M, p.K, dev->sm_count, desc->lhs_dt == RT_Q8_0H ? 2 : 4, gemv_split, pl->nv2 > 0);
         pl->split = gemv_split | wide << 8;
         pl->launches = 1 + (pl->nv2 > 0 ? 1 : 0);
         pl->name = std::string("q8_gemv_mma_") + (desc->lhs_dt == RT_Q8_0H ? "h" : "f") + "_nv" + std::to_string(pl->nv) +

@@ -68,8 +68,8 @@ __device__ __forceinline__ float scale_to_f32(float s) { return s; }
 __host__ __device__ inline int code_row_stride(int ks) { return ks + ((32 - ks % 128) + 128) % 128; }
 __host__ __device__ inline int scale_row_stride(int nblk_slice) { return nblk_slice | 1; }
 
-// Shared memory: [codes 16 x cstride][scales 16 x sstride][mbarrier]; the first 4 KB double as the
-// cross-warp reduction buffer once the codes have been consumed (the mbarrier lies beyond it).
+// Shared memory: [codes rows x cstride][scales rows x sstride][mbarrier]; the first WARPS x rows x cols floats (4 to 16 KB)
+// double as the cross-warp reduction buffer once the codes have been consumed (the mbarrier lies beyond it).
 __host__ __device__ inline size_t bar_offset(int blocks_per_cta, int scale_size, int cols, int rows) {
     const size_t codes = (size_t)rows * code_row_stride(blocks_per_cta * 32);
     const size_t scales = ((size_t)rows * scale_row_stride(blocks_per_cta) * scale_size + 15) & ~(size_t)15;
@@ -354,17 +354,41 @@ int q8_gemv_mma_pick_split(int M, int K, int sm_count, int scale_size) {
 // where the one-tile form needs several too.  16 vectors, us, one row tile -> two: [16384, 3072] 36.9 -> 23.1 (512 CTAs on 296
 // places, split 1), [3072, 8192] 21.3 -> 13.1 (384 on 444, split 4), [3072, 1024] 7.5 -> 4.9, [1536, 3072] 8.2 -> 6.3; but
 // [10240, 2560] 13.6 -> 17.4 (320 CTAs on 296 places) and [2560, 10240] 16.3 -> 19.9, whose one-tile form is one wave.
-int q8_gemv_mma_pick_wide(int M, int K, int sm_count, int scale_size, int split) {
+// The split in one wave (us, splits 1 / 2 / 4 / 8): rows of up to about 5000 values are not split, a cluster costs more than it
+// shortens them ([2912, 3936] x 15 8.8 / 9.7 / 9.2, one row tile 14.7; [1760, 4736] x 15 7.3 / 7.7, one 9.1); longer ones are
+// ([1600, 6208] x 16 10.5 / 9.2 / 9.2, one 10.7), and shorter ones where there are few of them ([640, 4064] x 14 6.7 / 6.7 / 6.2,
+// one 6.4) or where the second pass of 17..24 vectors brings clusters of eight ([1280, 4384] x 24 16.6 / 16.2 / 14.8, one 15.4).
+// Once a cluster is paid for it grows until a CTA is on every SM ([640, 12288] x 9 - / 9.5 / 7.9 / 8.1, one 8.5).
+int q8_gemv_mma_pick_wide(int M, int K, int sm_count, int scale_size, int split, bool two_passes) {
     const int nblk = K / 32;
     auto places = [&](int rows, int s, int by_regs) {
         const size_t smem = smem_bytes((nblk + s - 1) / s, scale_size, 16, rows) + 1024; // the system's own share per CTA
         return smem > 228 * 1024 ? 0 : sm_count * (int)std::min<size_t>(by_regs, 228 * 1024 / smem);
     };
-    const int groups = (M + 2 * ROWS - 1) / (2 * ROWS);
-    for (int s = 1; s <= 8 && (s == 1 || nblk / s >= 2 * WARPS); s *= 2)
-        if (groups * s <= places(2 * ROWS, s, 3)) return s;
+    const int groups = (M + 2 * ROWS - 1) / (2 * ROWS), one = (M + ROWS - 1) / ROWS * split; // row groups; CTAs of the one-tile form
+    auto one_wave = [&](int s) { return (s == 1 || nblk / s >= 2 * WARPS) && groups * s <= places(2 * ROWS, s, 3); };
+    const int longest = 6 * groups <= sm_count || (two_passes && split == 8) ? 124 : 164; // blocks of a row in one CTA
+    int pick = 0;
+    for (int s = 1; s <= 8; s *= 2)
+        if (one_wave(s) && (!pick || (nblk + pick - 1) / pick > longest)) pick = s;
+    if (pick > 0) {
+        const int full = two_passes ? sm_count * 9 / 8 : sm_count;
+        while (pick > 1 && pick < 8 && groups * pick * 2 <= full && one_wave(pick * 2)) pick *= 2;
+        // With at most one CTA on an SM in the one-tile form two row tiles only take longer, unless they do without its cluster:
+        // [1152, 448] x 9 3.10 -> 3.35, [512, 832] x 9 3.36 -> 3.48, [288, 6272] x 17 10.0 -> 10.1 at the best split; but
+        // [384, 1536] x 16 (split 2 -> 1) 5.66 -> 4.89.
+        if (one <= sm_count && (split == 1 || pick > 1)) return 0;
+        // Rows of a few blocks per warp, up to three CTAs per SM: a launch takes what its fullest SM takes ([5568, 672] x 14, 64 rows
+        // there instead of 48: 5.16 -> 5.40), and the shortest gain nothing from equal shares ([3648, 480] x 22 7.19 -> 7.45,
+        // [2304, 448] x 16 5.64 -> 5.94); [6528, 864] x 10 gains from 64 instead of 48 (7.34 -> 7.07), [4320, 576] x 24 from
+        // equal shares (8.52 -> 8.06), [5056, 704] x 24, whose second pass follows, from 64 instead of 48 (11.7 -> 10.6).
+        const int rows2 = (groups + sm_count - 1) / sm_count * 2, rows1 = (one + sm_count - 1) / sm_count; // of the fullest SM / 16
+        if (split == 1 && one <= 3 * sm_count &&
+            (nblk < 2 * WARPS ? rows2 >= rows1 : nblk < 3 * WARPS && rows2 > rows1 && !two_passes)) return 0;
+        return pick;
+    }
     const int room1 = places(2 * ROWS, 1, 3), room_one_tile = places(ROWS, split, 5);
-    if (room1 > 0 && room_one_tile > 0 && (M + ROWS - 1) / ROWS * split > room_one_tile) {
+    if (room1 > 0 && room_one_tile > 0 && one > room_one_tile) {
         const int waves = (groups + room1 - 1) / room1;
         if (5 * groups >= 4 * waves * room1) return 1;
     }

@@ -61,7 +61,8 @@ cudaError_t launch_rowvec_mat(const MatmulParams &p, rt_dtype dt, int chunks, fl
 // lhs_constant: the weight bytes are not written by any work in flight on the stream, so the
 // kernel may request them before it waits for its stream predecessor.
 int q8_gemv_mma_pick_split(int M, int K, int sm_count, int scale_size);
-int q8_gemv_mma_pick_wide(int M, int K, int sm_count, int scale_size, int split); // two row tiles per CTA for 9..16 vectors: its K split, or 0
+// two row tiles per CTA for 9..16 vectors: its K split, or 0; two_passes: a second launch takes vectors 17..24
+int q8_gemv_mma_pick_wide(int M, int K, int sm_count, int scale_size, int split, bool two_passes);
 cudaError_t launch_q8_gemv_mma(const MatmulParams &p, bool f32_scales, int nv, int split, bool lhs_constant, cudaStream_t stream);
 cudaError_t gemv_bind_wait_error(int *word);
 

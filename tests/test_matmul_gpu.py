@@ -1225,3 +1225,37 @@ def test_q4k_f16_gemv_with_a_nan_is_no_slower_than_the_staging_kernel(gpu, monke
         b.synchronize()
         took.append(a.elapsed_time(b))
     assert took[0] <= 1.2 * took[1], took
+
+
+@pytest.mark.parametrize("N,K,rows,form", [
+    (16384, 3072, 16, "nv16_split1_rows32"),
+    (3072, 8192, 16, "nv16_split4_rows32"),
+    (2560, 2560, 16, "nv16_split1_rows32"),   # the one-tile form would need a cluster of four
+    (10240, 2560, 16, "nv16_split1"),         # 320 CTAs of two row tiles on 296 places
+    (2560, 10240, 16, "nv16_split4"),
+    (640, 12288, 16, "nv16_split4_rows32"),   # long rows, few of them: split until a CTA is on every SM
+    (640, 4064, 14, "nv14_split4_rows32"),
+    (1600, 6208, 24, "nv16+8_split2_rows32"),
+    (1280, 4384, 16, "nv16_split1_rows32"),
+    (1280, 4384, 21, "nv16+5_split4_rows32"),
+    (384, 11488, 12, "nv12_split8_rows32"),
+    (288, 6272, 17, "nv16+1_split8"),         # one CTA per SM in the one-tile form
+    (1152, 448, 9, "nv9_split1"),
+    (512, 832, 9, "nv9_split1"),
+    (5568, 672, 14, "nv14_split1"),           # two CTAs of 32 rows on the fullest SM against three of 16
+    (3648, 480, 22, "nv16+6_split1"),
+    (4320, 576, 24, "nv16+8_split1_rows32"),
+])
+def test_q8_skinny_form_follows_the_measured_rule(gpu, N, K, rows, form):
+    node = Tensor([N, K], Q8H, gpu, None).gemm(Tensor([1, rows, K], F16, gpu, None), None, False, True, True)
+    assert rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode() == "q8_gemv_mma_h_" + form
+
+
+@pytest.mark.parametrize("lhs_dt,N,K,rows,form", [
+    (Q8H, 1241, 5600, 16, "split2_rows32"),   # an uneven share of K, a last CTA of 25 rows
+    (Q8H, 645, 8192, 9, "split4_rows32"),
+    (Q8H, 391, 11488, 23, "split8_rows32"),   # the last rank's share is shorter; a second pass of seven
+    (Q8F, 640, 6208, 13, "split4_rows32"),    # f32 scales
+])
+def test_q8_skinny_form_of_two_row_tiles_split_over_a_cluster_matches_the_oracle(gpu, lhs_dt, N, K, rows, form):
+    _check_linear(gpu, lhs_dt, F16, N, K, rows, True, 1, form)
