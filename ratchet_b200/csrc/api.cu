@@ -709,6 +709,8 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
     // short rows against very many of them (the Whisper logits, [51865, 384]): the 16-row CTAs of the streaming
     // kernel come to 3,242 tiny CTAs; the CUDA-core GEMV with 8 rows per warp is faster there (12.6 against 16.4 us)
     const bool short_rows = q8 && s.N == 1 && s.K <= 512 && s.M >= 16384 && s.K % 32 == 0;
+    // the warp-MMA Q4_K kernel's launch shape for one vector (0: rows too long for its shared memory)
+    const int q4k_one = desc->lhs_dt == RT_Q4_K && s.N == 1 && !empty ? q4k_gemv_pick_split(p.M, p.K, 1, (int)s.stacks, dev->sm_count) : 0;
     if (gemv_split > 0 && !short_rows && desc->rhs_dt == RT_F16 && !s.trans_lhs && s.N >= 1 && s.N <= 8 && (s.N == 1 || s.trans_rhs) && s.K > 0 && !empty) {
         pl->nv = (int)s.N;
         pl->split = gemv_split;
@@ -748,11 +750,14 @@ static rt_status build_plan(rt_device *dev, const rt_matmul_desc *desc, rt_plan 
                    (pl->nv2 ? "+" + std::to_string(pl->nv2) : std::string()) + "_split" + std::to_string(wide ? wide : gemv_split) +
                    (wide ? "_rows32" : "");
     } else if (desc->lhs_dt == RT_Q4_K && desc->rhs_dt == RT_F16 && !s.trans_lhs && s.N == 1 && s.K > 0 && s.K % 256 == 0 && !empty && !force_simt() &&
-               getenv("RT_Q4K_UMMA") == nullptr && !(s.K > 2048 && (q4k_gemv_pick_split(p.M, p.K, 1, (int)s.stacks, dev->sm_count) & 0xff) == 1)) {
+               getenv("RT_Q4K_UMMA") == nullptr && !(s.K > 2048 && (q4k_one & 0xff) == 1) && (q4k_one > 0 || s.epilogue != RT_EPILOGUE_SILU_MUL)) {
         // one vector: registers only (RT_Q4K_UMMA=1 / 0 picks the tensor-memory or the warp-MMA kernel instead).  The warp-MMA
         // kernel keeps the long rows of which one CTA holds all K and which fill the machine without a K split:
         // [10240, 2560] 11.0 against 11.8 us, [16384, 3072] with the fold 16.8 against 17.8.
+        // Rows too long for the warp-MMA kernel belong to the general one where operands are not 16-byte aligned, which it
+        // takes as they are (launch_node); with the fold it has those rows alone, since only its plan has the fold's scratch.
         pl->kernel = PK_Q4K_GEMV_F16;
+        pl->split = q4k_one;
         pl->name = "q4k_gemv_f16";
     } else if (desc->lhs_dt == RT_Q4_K && desc->rhs_dt == RT_F16 && !s.trans_lhs && s.N >= 1 && s.N <= 16 &&
                (s.N == 1 || s.trans_rhs) && !empty && !force_simt() && s.stacks == 1 && q4k_umma_enabled() &&
@@ -1104,8 +1109,11 @@ static rt_status launch_node(rt_plan *plan, const void *lhs, const void *rhs, co
         }
         break;
     case PK_Q4K_GEMV_F16:
-        if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) % 16 != 0)
-            return fail(RT_ERR_ARG, "rt_matmul_launch: lhs and rhs must be 16-byte aligned");
+        if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(rhs)) % 16 != 0) {
+            if (plan->split > 0) return fail(RT_ERR_ARG, "rt_matmul_launch: lhs and rhs must be 16-byte aligned");
+            e = launch_matmul_simt(p, s.desc.lhs_dt, s.desc.rhs_dt, true, st);
+            break;
+        }
         e = launch_q4k_gemv_f16(p, s.epilogue == RT_EPILOGUE_SILU_MUL, (flags & RT_LAUNCH_LHS_CONSTANT) != 0, st);
         break;
     case PK_Q4K_GEMV:

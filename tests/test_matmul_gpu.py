@@ -1259,3 +1259,27 @@ def test_q8_skinny_form_follows_the_measured_rule(gpu, N, K, rows, form):
 ])
 def test_q8_skinny_form_of_two_row_tiles_split_over_a_cluster_matches_the_oracle(gpu, lhs_dt, N, K, rows, form):
     _check_linear(gpu, lhs_dt, F16, N, K, rows, True, 1, form)
+
+
+@pytest.mark.parametrize("K,fold,kernel", [(131072, False, "q4k_gemv_f16"), (131072, True, "gemv_simt_Q4_K_F16+silu_mul"), (4096, False, "q4k_gemv_f16")])
+def test_q4k_one_vector_that_is_not_16_byte_aligned(gpu, K, fold, kernel):
+    """Rows too long for the staging kernel were always the general kernel's, which takes operands as they lie; shorter ones
+    are refused before anything is launched."""
+    lib, N = rb._lib.load(), 16
+    w_t, wv = make_lhs(Q4K, (N, K), np.random.default_rng(3), 0.02)
+    x = np.random.default_rng(4).standard_normal((1, 1, K)).astype(np.float16)
+    w_d, x_d = w_t.to(gpu), Tensor.from_data(np.concatenate([np.zeros(1, np.float16), x.reshape(-1)]), gpu)
+    node = w_d.gemm(Tensor([1, 1, K], F16, gpu, None), None, False, True, True, epilogue=rb.EPILOGUE_SILU_MUL if fold else 0)
+    plan = gpu.plan_for(node.op.desc)
+    assert lib.rt_plan_kernel(plan).decode() == kernel
+    out = Tensor(node.shape, F16, gpu, rb.GpuBuffer(gpu, 2 * node.numel()))
+    status = lib.rt_matmul_launch(plan, w_d.ptr, x_d.ptr + 2, None, out.ptr, None)
+    if K == 4096:
+        assert status == rb._lib.RT_ERR_ARG and b"16-byte aligned" in lib.rt_last_error()
+        return
+    rb._lib.check(status)
+    gpu.sync()
+    want = oracle.f64_to_f16(wv.reshape(N, K).astype(np.float64) @ x.reshape(-1).astype(np.float64)).astype(np.float32)
+    if fold:
+        want = want[N // 2:] * (want[:N // 2] / (1 + np.exp(-want[:N // 2])))
+    assert oracle.rel_l2(out.to(Device.CPU).to_f32().reshape(-1), want) <= TOL[F16]
