@@ -162,7 +162,7 @@ static std::string routing_switches() {
     for (const char *name : ROUTING_SWITCHES) {
         const char *v = getenv(name);
         k += '|';
-        if (v) k += v;
+        if (v) (k += '=') += v; // (some switches tell an empty value from none)
     }
     return k;
 }

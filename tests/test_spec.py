@@ -345,3 +345,17 @@ def test_plans_kept_per_device_are_bounded(monkeypatch):
     for stamp in range(2 * form.LIMIT + 3):
         form.plan(device, stamp)
     assert len(device._form_plans) <= form.LIMIT
+
+
+@pytest.mark.parametrize("switch", ["RT_Q4K_UMMA", "RT_GEMM_KSPLIT"])
+def test_a_routing_switch_set_to_nothing_is_told_from_an_unset_one(monkeypatch, switch):
+    """Routing takes them differently, so plans made under one must not be handed out under the other."""
+    stamp = _lib.load().rt_routing_stamp
+    monkeypatch.delenv(switch, raising=False)
+    unset = stamp()
+    monkeypatch.setenv(switch, "")
+    empty = stamp()
+    monkeypatch.setenv(switch, "0")
+    assert len({unset, empty, stamp()}) == 3
+    monkeypatch.delenv(switch)
+    assert stamp() == unset
