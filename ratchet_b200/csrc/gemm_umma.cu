@@ -30,6 +30,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "asked_once.hpp"
 #include "common.cuh"
 #include "kernels.hpp"
 #include "wait_error.cuh"
@@ -958,37 +959,34 @@ cudaError_t launch_ksplit(const CUtensorMap &mp, const CUtensorMap &mq, UmmaPara
     return cudaLaunchKernelEx(&lc, kernel, mp, mq, prm, ksplit);
 }
 
-// Clusters of `ksplit` such CTAs that the current device holds at once (0: none); asked once per device and size.
+// Clusters of `ksplit` such CTAs that the current device holds at once (0: none, or it could not be asked).
 int ksplit_capacity(int ksplit) {
-    static std::mutex mu;
-    static std::unordered_map<int, int> known;
+    static AskedOnce capacities;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    std::lock_guard<std::mutex> lk(mu);
-    const int key = dev * 16 + ksplit;
-    auto it = known.find(key);
-    if (it != known.end()) return it->second;
-    auto kernel = gemm_umma_ksplit_kernel<256, __half, false, 8>;
-    int n = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<256>::SMEM_BYTES) == cudaSuccess) {
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3((unsigned)ksplit * 148);
-        lc.blockDim = dim3(NUM_THREADS);
-        lc.dynamicSmemBytes = KsCfg<256>::SMEM_BYTES;
+    // either tile width takes one CTA per SM, so one instantiation answers for both
+    static_assert(2 * KsCfg<128>::SMEM_BYTES > 228 * 1024 && 2 * KsCfg<256>::SMEM_BYTES > 228 * 1024, "one CTA per SM");
+    return capacities.get(dev * 16 + ksplit, [&] {
+        auto kernel = gemm_umma_ksplit_kernel<256, __half, false, 8>;
+        int n = 0, sms = 0;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)ksplit;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc = {};
+        lc.blockDim = dim3(NUM_THREADS);
+        lc.dynamicSmemBytes = KsCfg<256>::SMEM_BYTES;
         lc.attrs = attr;
         lc.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &lc) != cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
-    }
-    known[key] = n;
-    return n;
+        cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        lc.gridDim = dim3((unsigned)(ksplit * sms));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KsCfg<256>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kernel, &lc);
+        if (e == cudaSuccess) return n;
+        cudaGetLastError();
+        return -1;
+    });
 }
 
 // The output as the epilogue's TMA stores see it: [stacks][R][columns up to the end of this launch's window].

@@ -2,6 +2,7 @@
 import ctypes
 import os
 import re
+import subprocess
 from ctypes import byref
 
 import numpy as np
@@ -359,3 +360,24 @@ def test_a_routing_switch_set_to_nothing_is_told_from_an_unset_one(monkeypatch, 
     assert len({unset, empty, stamp()}) == 3
     monkeypatch.delenv(switch)
     assert stamp() == unset
+
+
+def test_a_device_question_that_failed_is_asked_again(tmp_path):
+    """The cluster capacities behind the K split are asked once; one failure must not switch a cluster size off for good."""
+    (tmp_path / "t.cpp").write_text("""
+        #include "asked_once.hpp"
+        int main() {
+            rt::AskedOnce a;
+            int asked = 0, answer = -1;
+            auto ask = [&] { asked++; return answer; };
+            if (a.get(3, ask) != 0 || asked != 1) return 1;
+            answer = 74;
+            if (a.get(3, ask) != 74 || asked != 2) return 2;
+            answer = 5;
+            if (a.get(3, ask) != 74 || asked != 2) return 3;
+            answer = 0;
+            return a.get(4, ask) != 0 || a.get(4, ask) != 0 || asked != 3 ? 4 : 0;
+        }""")
+    csrc = os.path.join(ROOT, "ratchet_b200", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-I", csrc, str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
