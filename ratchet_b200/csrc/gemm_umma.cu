@@ -1099,6 +1099,10 @@ void umma_pick_tile(long long R, long long S, long long K, long long stacks, boo
         }
 }
 
+void umma_ask_capacities() {
+    for (int split = 2; split <= UMMA_KSPLIT_MAX; split++) ksplit_capacity(split);
+}
+
 // P: [p_stack][R][K] of p_dt, Q: [q_stack][S][K] of q_dt (f16 or bf16 each); out [stacks][R][S] of out_dt.
 cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dtype q_dt, void *out, rt_dtype out_dt,
                              int R, int S, int K, int stacks, int p_stack, int q_stack, const void *bias, int bias_dt,

@@ -123,6 +123,7 @@ constexpr int UMMA_BN_PAIR = 512;
 int umma_pick_bn(long long R, long long S, long long stacks, int sm_count);
 // K split over the CTAs of a cluster (portable cluster sizes), for problems with fewer tiles than SMs
 constexpr int UMMA_KSPLIT_MAX = 8;
+void umma_ask_capacities(); // what umma_pick_tile asks the current device, for callers that must not ask later
 void umma_pick_tile(long long R, long long S, long long K, long long stacks, bool pair, int sm_count, int *bn, int *ksplit);
 cudaError_t launch_gemm_umma(const void *P, rt_dtype p_dt, const void *Q, rt_dtype q_dt, void *out, rt_dtype out_dt,
                              int R, int S, int K, int stacks, int p_stack, int q_stack, const void *bias, int bias_dt,

@@ -61,6 +61,7 @@ extern "C" rt_status rt_linear_q8_0_static_scratch(rt_device *dev, const void *w
             e = cudaGetSymbolAddress(&p, g_static_scratch);
             if (e != cudaSuccess || !p)
                 return fail(RT_ERR_CUDA, std::string("cudaGetSymbolAddress(static scratch): ") + cudaGetErrorString(e));
+            umma_ask_capacities();
             g_scratch_addr[ordinal] = p;
         }
         scratch = g_scratch_addr[ordinal];
@@ -74,8 +75,8 @@ extern "C" rt_status rt_linear_q8_0_static_scratch(rt_device *dev, const void *w
     // tensor map stops at n*k: nothing left over from an earlier call is ever read, nothing needs zeroing
     e = launch_dequant(RT_Q8_0H, (long long)numel, w, scales, scratch, RT_F16, sm_count, st);
     if (e == cudaSuccess) {
-        int bn = 128, ksplit = 1; // the regular route's choice: the same bits
-        umma_pick_tile(rows, n, k, 1, epilogue == RT_EPILOGUE_SILU_MUL, sm_count, &bn, &ksplit);
+        int bn = 128, ksplit = 1; // the regular route's choice (CTA pairs add in the same order): the same bits
+        umma_pick_tile(rows, n, k, 1, false, sm_count, &bn, &ksplit);
         e = launch_gemm_umma(x, RT_F16, scratch, RT_F16, out, RT_F16, (int)rows, (int)n, (int)k, 1, 1, 1, bias, RT_F16,
                              bias ? BIAS_PER_N : BIAS_NONE, epilogue, bn, sm_count, st, nullptr, nullptr, nullptr, ksplit);
     }

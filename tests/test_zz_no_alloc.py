@@ -96,3 +96,43 @@ def test_static_scratch_refuses_weights_beyond_its_array(gpu):
     assert st == _lib.RT_ERR_ARG
     st = lib.rt_linear_q8_0_static_scratch(gpu._h, dummy.ptr, dummy.ptr + 4096 + 4, None, dummy.ptr + 8192, 16, 64, 64, 0, None)
     assert st == _lib.RT_ERR_ARG and b"16-byte aligned" in lib.rt_last_error()
+
+
+_CAPTURE = """
+import numpy as np, torch
+import ratchet_b200 as rb
+from ratchet_b200 import DType, Device, DeviceRequest, Quantizer, Quantization, Tensor, _lib
+gpu, lib, rng = Device.request_device(DeviceRequest.GPU), _lib.load(), np.random.default_rng(1)
+
+def operands(n, k, rows):
+    import oracle
+    w = Tensor.from_quantized(oracle.q8_quantize_h((rng.standard_normal((n, k)) * 0.02).astype(np.float32)), DType.Q8_0H, (n, k), gpu)
+    x = Tensor.from_data(rng.standard_normal((rows, k)).astype(np.float16), gpu)
+    out = Tensor([rows, n], DType.F16, gpu, rb.GpuBuffer(gpu, rows * n * 2))
+    return (w.ptr, x.ptr, None, out.ptr, rows, n, k, 0), (w, x, out)
+
+many, keep = operands(1536, 384, 1500)       # 144 tiles: no K split is considered
+few, (w, x, out) = operands(1024, 4096, 77)  # 8 tiles of 64 K blocks: split
+_lib.check(lib.rt_linear_q8_0_static_scratch(gpu._h, *many, None))
+gpu.sync()
+stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, stream=stream):
+    _lib.check(lib.rt_linear_q8_0_static_scratch(gpu._h, *few, stream.cuda_stream))
+graph.replay()
+torch.cuda.synchronize()
+got = out.to(Device.CPU).to_numpy().copy()
+node = w.gemm(x, None, False, True, True)
+assert "_ksplit" in lib.rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()
+assert np.array_equal(got.reshape(-1), node.resolve().to(Device.CPU).to_numpy().reshape(-1))
+print("CAPTURED")
+"""
+
+
+def test_after_the_first_call_on_a_device_a_shape_with_a_k_split_can_be_captured(gpu):
+    """The first call on a device does the set-up; later ones of any shape may be inside a stream capture."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CAPTURE], cwd=root, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0 and "CAPTURED" in r.stdout, r.stdout[-3000:]
