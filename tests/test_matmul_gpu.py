@@ -1283,3 +1283,96 @@ def test_q4k_one_vector_that_is_not_16_byte_aligned(gpu, K, fold, kernel):
     if fold:
         want = want[N // 2:] * (want[:N // 2] / (1 + np.exp(-want[:N // 2])))
     assert oracle.rel_l2(out.to(Device.CPU).to_f32().reshape(-1), want) <= TOL[F16]
+
+
+# ----------------------------------------------------------------------------- K split over a cluster: factors, windows, the default rule
+
+@pytest.mark.parametrize("lhs_dt", [Q8H, Q4K])
+@pytest.mark.parametrize("trans_out", [True, False])
+@pytest.mark.parametrize("split", ["128,3", "256,2"])
+def test_bf16_activations_outside_the_f16_range_with_k_split_over_a_cluster(gpu, monkeypatch, lhs_dt, trans_out, split):
+    """The row factors (trans_out) and the column factors go onto the summed accumulators."""
+    monkeypatch.setenv("RT_GEMM_KSPLIT", split)
+    node = Tensor([264, 512], lhs_dt, gpu, None).gemm(Tensor([1, 70, 512], BF16, gpu, None), None, False, True, trans_out)
+    assert "_ksplit" in rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()
+    test_bf16_activations_outside_the_f16_range_against_quantised_weights(gpu, lhs_dt, trans_out)
+
+
+def test_gate_up_fold_with_row_factors_and_k_split_over_a_cluster(gpu, monkeypatch):
+    monkeypatch.setenv("RT_GEMM_KSPLIT", "128,3")
+    _check_linear(gpu, Q8H, BF16, 1280, 512, 200, True, 2, "_bn128_ksplit3")
+
+
+@pytest.mark.parametrize("N,K,rows,widths,split,kernel_part", [
+    (1536, 4096, 77, [768, 768], None, "_ksplit"),           # the rule's own choice
+    (512, 1024, 200, [270, 242], "128,3", "_bn128_ksplit3"),  # windows that start and end inside four columns: single stores
+    (768, 640, 150, [256, 512], "256,5", "_bn256_ksplit5"),
+])
+def test_scattered_outputs_with_k_split_over_a_cluster(gpu, monkeypatch, N, K, rows, widths, split, kernel_part):
+    """Column windows of two full-width outputs, every element against the oracle; nothing outside a window is touched."""
+    from ctypes import byref
+    if split:
+        monkeypatch.setenv("RT_GEMM_KSPLIT", split)
+    lib = rb._lib.load()
+    w_t, wv = make_lhs(Q8H, (N, K), np.random.default_rng(31), 0.03)
+    b = round_to(F16, np.random.default_rng(32).standard_normal(N).astype(np.float32) * 0.1)
+    x = round_to(BF16, np.random.default_rng(33).standard_normal((rows, K)).astype(np.float32))
+    x_d = Tensor.from_data(x, gpu, BF16)
+    truth = oracle.matmul_truth(wv, x, b, 1, 1, 1, N, rows, K, False, True, True, 1).reshape(rows, N)
+    want = oracle.bf16_bits_to_f32(oracle.f64_to_bf16_bits(truth)).reshape(rows, N)
+    outs = [Tensor([rows, N], BF16, gpu, rb.GpuBuffer(gpu, rows * N * 2)) for _ in range(2)]
+    for o in outs:
+        o.write(np.full(rows * N, 0x7FC0, dtype=np.uint16))
+    c0 = 0
+    for wd in widths:
+        shard = rb.shard_rows(w_t, c0, c0 + wd).to(gpu)
+        bias = Tensor.from_data(np.ascontiguousarray(b[c0:c0 + wd]), gpu, F16)
+        plan = gpu.plan_for(shard.gemm(x_d, bias, False, True, True, epilogue=rb.EPILOGUE_GELU_TANH).op.desc)
+        assert kernel_part in lib.rt_plan_kernel(plan).decode(), lib.rt_plan_kernel(plan).decode()
+        opts = rb._lib.rt_launch_opts()
+        opts.flags, opts.n_out, opts.out_ld, opts.out_col = rb._lib.RT_LAUNCH_LHS_CONSTANT, 2, N, c0
+        opts.outs[0], opts.outs[1] = outs[0].ptr, outs[1].ptr
+        rb._lib.check(lib.rt_matmul_launch_ex(plan, shard.ptr, x_d.ptr, bias.ptr, None, None, byref(opts)))
+        gpu.sync()
+        c0 += wd
+        for o in outs:
+            got = o.to(Device.CPU).to_f32().reshape(rows, N)
+            assert oracle.rel_l2(got[:, :c0], want[:, :c0]) <= TOL[BF16] and np.all(np.isnan(got[:, c0:]))
+
+
+@pytest.mark.parametrize("lhs_dt,act,N,K,rows,part", [
+    (Q8H, F16, 2560, 10240, 77, "_ksplit"),
+    (F16, F16, 3072, 3072, 40, "_ksplit"),
+    (Q4K, F16, 3072, 8192, 512, "_bn256_ksplit2"),
+    (Q8H, F16, 10240, 2560, 128, "_bn128_dequant"),   # 80 tiles: two shares of K each would not be resident together
+])
+def test_which_gemms_split_k_without_a_switch(gpu, lhs_dt, act, N, K, rows, part):
+    node = Tensor([N, K], lhs_dt, gpu, None).gemm(Tensor([1, rows, K], act, gpu, None), None, False, True, True)
+    name = rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()
+    assert part in name, name
+
+
+# ----------------------------------------------------------------------------- the row-scaled cast of long bf16 rows
+
+@pytest.mark.parametrize("K", [4128, 10240, 16416])
+def test_bf16_cast_of_rows_past_4096_values_matches_the_oracle(gpu, K):
+    """Four warps share a row: rows whose largest value, far outside f16's range, lies in the share of each of them, and a
+    row count that gives a team three rows and one team of the last block none.  16416 values no longer stay in registers."""
+    N, rows = 64, 4739
+    w_t, wv = make_lhs(Q8H, (N, K), np.random.default_rng(5), 0.03)
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal((rows, K), dtype=np.float32)
+    sampled = np.unique(np.concatenate([np.arange(8), [2367, 2368, 2369, 4735, 4736, 4737, 4738], rng.integers(0, rows, size=49)]))
+    for n, r in enumerate(sampled):
+        at = 8 * (32 * (n % 4) + int(rng.integers(0, 32))) + int(rng.integers(0, 8)) + 1024 * int(rng.integers(0, K // 1024))
+        x[r, at] = np.float32([3e5, -1e9, 2e20, 7e4][n // 4 % 4])
+        x[r] *= np.float32([1.0, 1e-12, 1e6][n // 16 % 3])
+    x = round_to(BF16, x)
+    node = w_t.to(gpu).gemm(Tensor.from_data(x.reshape(1, rows, K), gpu, BF16), None, False, True, True)
+    assert "gemm_umma_Q8_0H_BF16" in rb._lib.load().rt_plan_kernel(gpu.plan_for(node.op.desc)).decode()
+    got = node.resolve().to(Device.CPU).to_f32().reshape(rows, N)
+    assert np.all(np.isfinite(got))
+    truth = x[sampled].astype(np.float64) @ wv.reshape(N, K).astype(np.float64).T
+    want = oracle.bf16_bits_to_f32(oracle.f64_to_bf16_bits(truth)).reshape(len(sampled), N)
+    for n, r in enumerate(sampled):  # a final rounding that falls the other way is 2^-8 of one of 64 values: 5e-4 of the row
+        assert oracle.rel_l2(got[r], want[n]) <= 2 * TOL[BF16], r
