@@ -929,7 +929,7 @@ cudaError_t launch_bn(const CUtensorMap &mp, const CUtensorMap &mq, UmmaParams p
 template <int BN, typename OutT>
 cudaError_t launch_ksplit(const CUtensorMap &mp, const CUtensorMap &mq, UmmaParams prm, int ksplit, cudaStream_t stream) {
     using C = KsCfg<BN>;
-    if (ksplit < 2 || ksplit > UMMA_KSPLIT_MAX || ksplit > (prm.K + BK - 1) / BK) return cudaErrorInvalidValue;
+    if (ksplit < 2 || ksplit > UMMA_KSPLIT_MAX || ksplit > (prm.K + BK - 1) / BK || prm.bias_mode == BIAS_PER_M) return cudaErrorInvalidValue;
     static SmemAttr smem_attr[4];
     const bool wide = ksplit > 4;
     auto kernel = prm.pair ? (wide ? gemm_umma_ksplit_kernel<BN, OutT, true, 8> : gemm_umma_ksplit_kernel<BN, OutT, true, 4>)

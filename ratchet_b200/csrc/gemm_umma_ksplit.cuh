@@ -184,8 +184,6 @@ gemm_umma_ksplit_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_
                         }
                     acc[n][0] = s.x; acc[n][1] = s.y; acc[n][2] = s.z; acc[n][3] = s.w;
                 }
-                float row_bias = 0.f;
-                if (!PAIR && prm.bias_mode == BIAS_PER_M) row_bias = load_bias(prm.bias, prm.bias_dt, rg);
                 if (HAS_OPERAND_FACTORS<OutT>) {
                     if (prm.p_scale) {
                         const float f = __ldg(prm.p_scale + (long long)(b % prm.p_stack) * prm.R + rg);
@@ -208,8 +206,7 @@ gemm_umma_ksplit_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_
                         const OutT uv = epilogue_value<OutT>(acc[UNITS - 1][e], has_bias, has_bias ? bias_s[BN / 2 + ch * 4 + e] : 0.f, RT_EPILOGUE_NONE);
                         o[e] = silu_mul_value<OutT>(gv, uv);
                     } else {
-                        const float bias = prm.bias_mode == BIAS_PER_N ? bias_s[ch * 4 + e] : row_bias;
-                        o[e] = epilogue_value<OutT>(acc[0][e], has_bias, bias, prm.epilogue);
+                        o[e] = epilogue_value<OutT>(acc[0][e], has_bias, has_bias ? bias_s[ch * 4 + e] : 0.f, prm.epilogue);
                     }
                 }
                 const long long at = (long long)b * prm.out_batch_stride + (long long)rg * prm.out_ld + prm.out_col + col;
