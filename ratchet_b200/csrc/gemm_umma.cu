@@ -120,7 +120,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (*abort_flag) return false;
         if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
             *abort_flag = 1;
-            report_wait_error(site);
+            note_wait_error(site);
             return false;
         }
     }
@@ -601,6 +601,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     tc_fence_before();
     __syncthreads();
     if (*abort_flag) {
+        report_wait_error();
         // give copies that may still be in flight time to land before the CTA's memory is released
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);
@@ -816,6 +817,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_co
     __syncthreads();
     cluster_sync_all(); // neither CTA leaves while the other may still signal its barriers or read its shared memory
     if (*abort_flag) {
+        report_wait_error();
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);
     }

@@ -231,6 +231,7 @@ gemm_umma_ksplit_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_
     __syncthreads();
     cluster_sync_all(); // the peers have read this CTA's partial tile
     if (*abort_flag) {
+        report_wait_error();
         // give copies that may still be in flight time to land before the CTA's memory is released
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);

@@ -422,6 +422,7 @@ gemm_umma_tf32x3_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_
     tc_fence_before();
     __syncthreads();
     if (*abort_flag) {
+        report_wait_error();
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);
     }

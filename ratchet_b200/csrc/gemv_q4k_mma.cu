@@ -222,7 +222,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == WARPS_WALK ? 1 : 0) q4k_g
             while (!mbar_try_wait(bar, parity)) {
                 if ((unsigned long long)clock64() - t0 > WAIT_LIMIT_CYCLES) {
                     ok = false;
-                    report_wait_error(1);
+                    note_wait_error(1);
+                    report_wait_error();
                     break;
                 }
             }

@@ -26,7 +26,7 @@
 //  * weights flagged constant are requested before the kernel waits for its stream predecessor.
 // A block of activations that holds a NaN or an infinity has no digits: its products are formed in f32 from
 // the decoded weights instead, so that they come out as IEEE arithmetic gives them.
-// Every wait is bounded; on expiry the kernel sets a device flag, leaves its loops, frees tensor memory and
+// Every wait is bounded; on expiry the kernel notes the site (wait_error.cuh), leaves its loops, frees tensor memory and
 // returns; the next rt_device_sync reports it.
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -104,7 +104,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (*abort_flag) return false;
         if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
             *abort_flag = 1;
-            report_wait_error(site);
+            note_wait_error(site);
             return false;
         }
     }
@@ -462,7 +462,7 @@ q4k_gemv_umma_kernel(const __grid_constant__ CUtensorMap map_w, const Q4kUmmaPar
                              : "=r"(done) : "r"(bar_red) : "memory");
                 if (!done && wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
                     *abort_flag = 1;
-                    report_wait_error(9);
+                    note_wait_error(9);
                     break;
                 }
             }
@@ -484,6 +484,7 @@ q4k_gemv_umma_kernel(const __grid_constant__ CUtensorMap map_w, const Q4kUmmaPar
         }
     }
     if (*abort_flag) {
+        report_wait_error();
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);
     }

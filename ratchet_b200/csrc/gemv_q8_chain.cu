@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
                                 if (*abort_flag) break;
                                 if (wait_clock() - t0 > cp.poll_limit) {
                                     *abort_flag = 1;
-                                    report_wait_error(8);
+                                    note_wait_error(8);
                                     break;
                                 }
                             }
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
                                 if (*abort_flag) break;
                                 if (wait_clock() - t0 > cp.poll_limit) {
                                     *abort_flag = 1;
-                                    report_wait_error(7);
+                                    note_wait_error(7);
                                     break;
                                 }
                             }
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
                                     if (*abort_flag) break;
                                     if (wait_clock() - t0 > cp.poll_limit) {
                                         *abort_flag = 1;
-                                        report_wait_error(7);
+                                        note_wait_error(7);
                                         break;
                                     }
                                 }
@@ -578,6 +578,7 @@ __global__ void __launch_bounds__(THREADS, 1) q8_gemv_chain_kernel(const ChainPa
     tc_fence_before();
     __syncthreads();
     if (*abort_flag) {
+        report_wait_error();
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);
     }

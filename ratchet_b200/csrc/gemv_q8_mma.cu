@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(THREADS, RT == 2 ? 3 : 5) q8_gemv_bulk_kernel(
         while (!mbar_try_wait(bar_addr, 0)) {
             if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
                 ok = false;
-                report_wait_error(1);
+                note_wait_error(1);
+                report_wait_error();
                 break;
             }
         }

@@ -27,7 +27,7 @@
 //    memory, so the next layer's CTAs are resident with their first stages loaded while this layer
 //    computes.  (Asking for the whole share with cp.async.bulk.prefetch.L2 as well measured 3 %
 //    slower: the requests compete with the running layer's refills.)
-// Every wait is bounded (about two seconds of SM cycles); on expiry the kernel sets a device flag,
+// Every wait is bounded (about two seconds of SM cycles); on expiry the kernel notes the site (wait_error.cuh),
 // leaves its loops, frees tensor memory and returns; the next rt_device_sync reports it.
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -289,7 +289,7 @@ q8_gemv_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                              : "=r"(done) : "r"(bar_red) : "memory");
                 if (!done && wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
                     *abort_flag = 1;
-                    report_wait_error(7);
+                    note_wait_error(7);
                     break;
                 }
             }
@@ -306,6 +306,7 @@ q8_gemv_umma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         ((__half *)p.out)[row] = epilogue_value<__half>(red[threadIdx.x], has_bias, bias, p.epilogue);
     }
     if (*abort_flag) {
+        report_wait_error();
         const unsigned long long t0 = wait_clock();
         while (wait_clock() - t0 < 400000ull) __nanosleep(1000);
     }

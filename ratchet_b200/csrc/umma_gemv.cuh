@@ -47,7 +47,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: gives up after WAIT_LIMIT_CYCLES, or as soon as the CTA's abort flag is up; the
-// site that gives up is reported to the host, which looks at its next sync.
+// first site that gives up is noted, and reported by its CTA on the way out (wait_error.cuh).
 __device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, volatile int *abort_flag, int site) {
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = wait_clock();
@@ -58,7 +58,7 @@ __device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, vo
         if (*abort_flag) return false;
         if (wait_clock() - t0 > WAIT_LIMIT_CYCLES) {
             *abort_flag = 1;
-            report_wait_error(site);
+            note_wait_error(site);
             return false;
         }
     }
