@@ -853,7 +853,9 @@ def test_gemm_on_cta_pairs_matches_the_oracle_and_the_single_cta_kernel(gpu, mon
 def test_scattered_outputs_on_one_gpu(gpu, N, K, rows, widths, kernel_part):
     """The N-sharded prefill form with every shard on ONE GPU: each shard's GEMM writes its column window into TWO
     full-width output buffers (rt_matmul_launch_ex with n_out = 2, the peer-store epilogue with local "peers").  Both
-    buffers end up holding the unsharded Linear's result, bit for bit, and nothing outside a window is touched."""
+    buffers end up holding the unsharded Linear's result and nothing outside a window is touched.  Bit for bit because
+    neither the whole nor a shard of these sizes has its K split: the split follows the number of columns (see
+    test_scattered_outputs_with_k_split_over_a_cluster)."""
     from ctypes import byref
     lib = rb._lib.load()
     w_t, wv = make_lhs(Q8H, (N, K), np.random.default_rng(31), 0.03)
